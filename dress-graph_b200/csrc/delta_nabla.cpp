@@ -10,8 +10,8 @@
 // histogram, edgeless subgraphs are skipped, and the histogram is the exact
 // (value, count) list ascending by value.
 //
-// Requests whose parent fits the batched kernel (rows of at most 31
-// neighbours, per-subgraph state within shared memory) are packed into one
+// Requests whose parent fits the batched kernel (one subgraph's state within
+// shared memory) are packed into one
 // persistent launch; any other request runs through the per-subgraph path:
 // host-built subgraph + single-graph GPU fit (the reference's structure,
 // which is also the "plain per-fit launch loop" the batched engine is
@@ -120,6 +120,165 @@ void merge_walk_pairs(p_dress_graph_t g, std::vector<int> &ioff, std::vector<int
 
 namespace {
 
+// High words that every live product of a subgraph must have for the batch
+// kernel's FastSum (batch.cu) to give the reference's bits, for any item:
+//   * below PHI, so that no term's exponent is above the sum's: a vertex sum
+//     starts at 4 nw >= A, an edge sum at twice that (once, in the FORWARD and
+//     BACKWARD variants) and its terms are sums of two products;
+//   * at least PLO, a power of two with n a 2^-50 < PLO for the longest item's
+//     n terms and a bound a on any sum: every term, partial sum and rounding
+//     error is then a multiple of ulp(PLO) and every sum of errors is below
+//     2^53 of them, so the additions of errors are exact in any order.
+// PHI is 4 nw rounded down to a power of two, doubled (unit weights: products
+// below 8), PLO about 2^-41 n^2: only products of zero or of values far from
+// any fixed point are outside.  All in units of the weight where that is one
+// power of two.  span = 0: no fast path.
+void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageShape &s)
+{
+    s.lo = s.span = 0;
+    const double unit = s.uniform ? s.wc : 1.0;
+    const double A = 4.0 * nw_min / unit, Amax = 4.0 * nw_max / unit;
+    if (!(A >= 0x1p-300) || !(Amax <= 0x1p300)) return;
+    const double phi = std::ldexp(1.0, std::ilogb(A) + (fwd ? 0 : 1));
+    const double n = most_terms;
+    const double bound = 2.0 * Amax + 2.0 * (n + 1.0) * phi;
+    const double plo = std::ldexp(1.0, std::ilogb(n * bound * 0x1p-50) + 1);
+    if (!(plo < phi)) return;
+    uint64_t b0, b1;
+    std::memcpy(&b0, &plo, 8);
+    std::memcpy(&b1, &phi, 8);
+    s.lo = (unsigned)(b0 >> 32);
+    s.span = (unsigned)(b1 >> 32) - s.lo;
+}
+
+}  // namespace
+
+ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind, int k, bool has_nw, bool has_dinit)
+{
+    const int N = g->N, E = g->E;
+    ImageShape s;
+    s.has_nw = has_nw;
+    s.has_dinit = has_dinit;
+    int most = 1;
+    for (int u = 0; u < N; ++u) {
+        const int q = (g->adj_offset[u + 1] - g->adj_offset[u] + 3) / 4;
+        s.Q += q;
+        most = std::max(most, 4 * q + 1);
+    }
+    for (int e = 0; e < E; ++e) {
+        const int p = (ioff[(size_t)e + 1] - ioff[(size_t)e] + 1) / 2;
+        s.P2 += p;
+        most = std::max(most, 2 * p + 1);
+    }
+    s.wc = 1.0;
+    if (E > 0) {
+        int ex = 0;
+        const double w0 = g->edge_weight[0];
+        bool same = w0 > 0.0 && std::isfinite(w0) && std::frexp(w0, &ex) == 0.5 && std::abs(ex) <= 300;
+        for (int e = 1; e < E && same; ++e) same = g->edge_weight[e] == w0;
+        s.uniform = same;
+        if (same) s.wc = w0;
+    } else {
+        s.uniform = 1;
+    }
+    double lo = 1.0, hi = 1.0;
+    if (kind == ITEM_PLAIN && has_nw && N > 0) {
+        lo = hi = g->NW[0];
+        for (int u = 1; u < N; ++u) {
+            lo = g->NW[u] < lo ? g->NW[u] : lo;
+            hi = g->NW[u] > hi ? g->NW[u] : hi;
+            if (std::isnan(g->NW[u])) lo = g->NW[u];
+            if (std::isnan(lo)) break;
+        }
+    } else if (kind == ITEM_NABLA && k > 0) {
+        hi = std::sqrt((double)std::max(53, 2 * k + 1));      // no marker weight is larger
+    }
+    fast_range(lo, hi, most, g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD, s);
+    return s;
+}
+
+void pack_image(p_dress_graph_t g, const std::vector<int> &ioff, const std::vector<int> &pairs, const ImageShape &s,
+                unsigned char *dst)
+{
+    const int N = g->N, E = g->E;
+    const ImageLayout L = image_layout(N, E, s.Q, s.P2, s.uniform, s.has_nw, s.has_dinit);
+    unsigned *edge = (unsigned *)(dst + L.edge), *row = (unsigned *)(dst + L.row);
+    uint16_t *eid = (uint16_t *)(dst + L.eid), *pr = (uint16_t *)(dst + L.pairs);
+    uint16_t *vmap = (uint16_t *)(dst + L.vmap), *emap = (uint16_t *)(dst + L.emap);
+    // stable counting sorts by groups, most first; order[i] = the i-th item's id
+    std::vector<int> order((size_t)std::max(N, E)), at;
+    const auto by_groups = [&](int n, auto groups, uint16_t *map) {
+        int most = 0;
+        for (int i = 0; i < n; ++i) most = std::max(most, groups(i));
+        at.assign((size_t)most + 2, 0);
+        for (int i = 0; i < n; ++i) ++at[(size_t)(most - groups(i)) + 1];
+        for (size_t c = 1; c < at.size(); ++c) at[c] += at[c - 1];
+        for (int i = 0; i < n; ++i) {
+            const int p = at[(size_t)(most - groups(i))]++;
+            order[(size_t)p] = i;
+            map[i] = (uint16_t)p;
+        }
+    };
+    by_groups(E, [&](int e) { return (ioff[(size_t)e + 1] - ioff[(size_t)e] + 1) / 2; }, emap);
+    std::vector<int> eorder(order.begin(), order.begin() + E);
+    by_groups(N, [&](int u) { return (g->adj_offset[u + 1] - g->adj_offset[u] + 3) / 4; }, vmap);
+    size_t o = 0;
+    for (int i = 0; i < N; ++i) {
+        const int u = order[(size_t)i];
+        const unsigned first = (unsigned)(o / 4);
+        for (int q = g->adj_offset[u]; q < g->adj_offset[u + 1]; ++q) eid[o++] = emap[g->adj_edge_idx[q]];
+        while (o % 4) eid[o++] = (uint16_t)E;
+        row[i] = first | (unsigned)(o / 4) << 16;
+        if (s.has_nw) ((double *)(dst + L.nw))[i] = g->NW[u];
+    }
+    o = 0;
+    for (int i = 0; i < E; ++i) {
+        const int e = eorder[(size_t)i];
+        edge[2 * (size_t)i] = (unsigned)vmap[g->U[e]] | (unsigned)vmap[g->V[e]] << 16;
+        edge[2 * (size_t)i + 1] = ioff[(size_t)e + 1] > ioff[(size_t)e] ? (unsigned)(o / 4) : NO_PAIRS;
+        if (!s.uniform) ((double *)(dst + L.w))[i] = g->edge_weight[e];
+        if (s.has_dinit) ((double *)(dst + L.dinit))[i] = g->edge_dress[e];
+        if (ioff[(size_t)e + 1] == ioff[(size_t)e]) continue;
+        for (int q = 2 * ioff[(size_t)e]; q < 2 * ioff[(size_t)e + 1]; ++q) pr[o++] = emap[pairs[(size_t)q]];
+        while (o % 4) pr[o++] = (uint16_t)E;
+        pr[o - 1] |= 0x8000u;
+    }
+}
+
+// The work is divided so that every CTA slot of the device has some.  Up to two
+// subgraphs a warp, a subgraph gets more warps, as far as its edges fill them:
+// one subgraph's chain of sweeps is then what is waited for (3,480 subgraphs on
+// 4,736 warps: 211 us at a warp each, 144 us at two).  Chunks are half a slot's
+// share up to one round of a CTA's groups, and from eight rounds a slot up to
+// four rounds, at least four chunks a slot (an image is staged once a chunk).
+// Parents in order of size, largest first, so the last chunks to end are short.
+void build_chunks(const std::vector<ChunkSource> &src, int min_warps, int sms, int ctas, int smem,
+                  std::vector<Chunk> &chunks)
+{
+    const int cta = BATCH_SM_WARPS / ctas;
+    chunks.clear();
+    long long total = 0;
+    for (const ChunkSource &s : src) total += s.items;
+    std::vector<int> order(src.size());
+    for (size_t i = 0; i < src.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return src[(size_t)a].E > src[(size_t)b].E; });
+    const long long share = (total + ctas * sms - 1) / (ctas * sms);           // subgraphs a slot
+    for (int i : order) {
+        const ChunkSource &s = src[(size_t)i];
+        const int useful = std::max(1, std::min(cta, (s.E + 31) / 32));
+        int warps = min_warps;
+        if (share < 2 * cta) warps = std::max(warps, std::min(useful, 2 * cta / (int)std::max<long long>(share, 1)));
+        warps = std::min(warps, cta);
+        const Geometry q = chunk_geometry(s.N, s.E, s.k, s.img, batch_room(smem), cta, warps);
+        long long n = std::max<long long>(1, std::min<long long>((share + 1) / 2, q.groups));
+        if (share >= 8LL * q.groups) n = std::min<long long>(4, share / (4LL * q.groups)) * q.groups;
+        for (long long f = 0; f < s.items; f += n)
+            chunks.push_back({s.parent, (int)std::min(n, s.items - f), s.first + f, warps, 0});
+    }
+}
+
+namespace {
+
 int lcg15(unsigned int *s)
 {
     *s = *s * 1103515245u + 12345u;
@@ -164,6 +323,7 @@ struct Prep {
     bool empty = false;                // nothing to fit
     bool batchable = false;
     std::vector<int> ioff, pairs;      // common-neighbour pairs (parent numbering)
+    ImageShape img;                    // shape of the packed image
     int M = 0;
     double *ms_host = nullptr;         // multiset matrix (caller owns after return)
     std::vector<long long> values_host;  // per-subgraph path: values collected on the host
@@ -231,8 +391,8 @@ Status prepare(Prep &p)
     // lookup of DIRECTED graphs with repeated directed edges.
     // The batch kernel also needs one subgraph's state in shared memory;
     // rows of any length are summed there (certified sums, no networks).
-    p.batchable = !(dup && g->variant == DRESS_VARIANT_DIRECTED) &&
-                  batch_group_bytes(p.E, p.N, k, 32) <= BATCH_GROUP_BYTES_MAX;
+    p.batchable = !(dup && g->variant == DRESS_VARIANT_DIRECTED) && batch_fits(p.E, p.N, k);
+    if (p.batchable) p.img = plan_image(g, p.ioff, r->kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA, k, false, false);
     return Status::Ok();
 }
 
@@ -372,14 +532,14 @@ Status hist_of_host_values(std::vector<Prep *> &ps, cudaStream_t st, int sms)
 }
 
 // ---- batched path ------------------------------------------------------------------
+// A schedule: threads per subgraph, at least, and CTAs to an SM.
+constexpr int BATCH_CTAS = 2;
 struct Tune {
-    int gsize, groups;
-    int per_sm = 1;          // CTAs meant to share an SM (shared memory split between them)
+    int gsize;
+    int per_sm = BATCH_CTAS;
 };
 
-// Threads per subgraph by edge count (sweeps of a few hundred edges keep a
-// warp busy; larger subgraphs split across more warps), unless the autotuner
-// has measured this size class.
+// Size class of a batch, for the schedules that the autotuner measured.
 struct TuneKey {
     int e, n, M, k;
     bool operator<(const TuneKey &o) const
@@ -395,71 +555,24 @@ TuneKey tune_key(int maxE, int maxN, int M, int maxk)
     return {next_pow2(maxE), next_pow2(maxN), M, maxk};
 }
 
+// One warp per subgraph and two CTAs to an SM unless the autotuner has
+// measured the size class: where memory holds fewer subgraphs than warps, the
+// kernel gives each more of them (chunk_geometry).
 Tune pick_tune(int maxE, int maxN, int M, int maxk, const dressx_config_t &cfg)
 {
-    int gs = cfg.group_threads > 0 ? cfg.group_threads
-           : maxE <= 640 ? 32 : maxE <= 2048 ? 64 : maxE <= 8192 ? 128 : 256;
-    if (cfg.group_threads <= 0) {
-        std::lock_guard<std::mutex> lk(g_tuned_mu);
-        auto it = g_tuned.find(tune_key(maxE, maxN, M, maxk));
-        if (it != g_tuned.end()) return it->second;
-    }
-    int groups = 512 / gs;
-    if (gs > 32 && groups > 15) groups = 15;
-    return {gs, groups, 1};
-}
-
-// Groups per CTA and parent staging for a given group size: as many groups
-// as shared memory holds (at most `groups`), staging the parent unless that
-// halves the groups.  False when not even one group fits.
-bool shape_launch(BatchLaunch &L, const Tune &tu, long long smem_cap_full, long long smem_sm = 0)
-{
-    // two CTAs per SM split the SM's shared memory (each keeps ~1 KB of
-    // system and static shared memory)
-    const long long smem_cap = tu.per_sm == 2 && smem_sm > 0 ? smem_sm / 2 - 2048 : smem_cap_full;
-    L.min_ctas = tu.per_sm == 2 && smem_sm > 0 ? 2 : 1;
-    L.gsize = tu.gsize;
-    L.per_group = 0;
-    L.stage = 1;
-    L.groups = tu.groups;
-    while (L.groups > 1 && (long long)batch_smem_bytes(L) > smem_cap) --L.groups;
-    if ((long long)batch_smem_bytes(L) > smem_cap) {
-        L.stage = 0;
-        L.groups = tu.groups;
-        while (L.groups > 1 && (long long)batch_smem_bytes(L) > smem_cap) --L.groups;
-    }
-    if ((long long)batch_smem_bytes(L) > smem_cap) return false;
-    if (L.stage && L.groups * 2 < tu.groups) {
-        // staging leaves too few groups: read parents from L2 instead
-        BatchLaunch L2 = L;
-        L2.stage = 0;
-        L2.groups = tu.groups;
-        while (L2.groups > 1 && (long long)batch_smem_bytes(L2) > smem_cap) --L2.groups;
-        if (L2.groups > L.groups) L = L2;
-    }
-    return true;
-}
-
-// Chunks: a few rounds of subgraphs per CTA visit, requests in order; with
-// limit >= 0 only the first `limit` subgraphs of the whole batch.
-void build_chunks(const std::vector<Prep *> &ps, int groups, long long limit, std::vector<Chunk> &chunks)
-{
-    chunks.clear();
-    const int chunk_items = 4 * groups;
-    long long taken = 0;
-    for (size_t i = 0; i < ps.size(); ++i)
-        for (long long f = 0; f < ps[i]->items; f += chunk_items) {
-            if (limit >= 0 && taken >= limit) return;
-            int c = (int)std::min<long long>(chunk_items, ps[i]->items - f);
-            chunks.push_back({(int)i, c, f});
-            taken += c;
-        }
+    if (cfg.group_threads > 0) return {cfg.group_threads};
+    std::lock_guard<std::mutex> lk(g_tuned_mu);
+    auto it = g_tuned.find(tune_key(maxE, maxN, M, maxk));
+    return it != g_tuned.end() ? it->second : Tune{32};
 }
 
 // A packed, uploaded batch: parents, chunks, value and statistics buffers.
 struct BatchPlan {
     std::vector<Prep *> ps;
     BatchLaunch L{};
+    int maxE = 1, maxN = 1, maxk = 1, M = 2;
+    long long max_state = 0;                 // largest smallest-form state of the batch
+    int gsize = 32;                          // threads per subgraph, at least
     std::vector<ParentDesc> descs;
     std::vector<Chunk> chunks;
     std::vector<long long> val_base;
@@ -475,8 +588,7 @@ struct BatchPlan {
     HistResult hist;
     bool need_hist = false;
     float fit_ms = 0.f, hist_ms = 0.f;       // device time of the last run
-    long long smem_cap = 0, smem_sm = 0;
-    int tuned_per_sm = 1;                    // CTAs per SM the autotuner chose
+    int per_sm = BATCH_CTAS;                 // CTAs to an SM
     cudaGraphExec_t gexec = nullptr;         // captured fit stage (dressx_batch_capture)
     ~BatchPlan()
     {
@@ -484,30 +596,56 @@ struct BatchPlan {
     }
 };
 
+// CTAs to an SM of a schedule, and their shared memory: one where a subgraph
+// needs more than half of an SM.  False when the schedule cannot run.
+Status shape_launch(BatchPlan &P, const Ctx &en, const Tune &tu, bool &fits)
+{
+    fits = true;
+    P.gsize = std::max(32, std::min(512, tu.gsize));
+    for (P.per_sm = tu.per_sm; P.per_sm >= 1; P.per_sm /= 2) {
+        P.L.ctas = P.per_sm;
+        DRESS_TRY(batch_smem(en.device, P.per_sm, &P.L.smem));
+        if (P.max_state <= batch_room(P.L.smem)) return Status::Ok();
+    }
+    fits = false;
+    return Status::Ok();
+}
+
+// The chunks of the whole batch, uploaded.
+Status chunk_batch(BatchPlan &P, const Ctx &en, DevBuf<Chunk> &dev, std::vector<Chunk> &chunks, BatchLaunch &L)
+{
+    std::vector<ChunkSource> src;
+    for (size_t i = 0; i < P.ps.size(); ++i)
+        src.push_back({(int)i, P.ps[i]->N, P.ps[i]->E, P.ps[i]->r->k, 0, P.ps[i]->items, P.ps[i]->img});
+    build_chunks(src, P.gsize / 32, en.num_sms, L.ctas, L.smem, chunks);
+    DRESS_TRY(dev.alloc(chunks.size(), en.st));
+    DRESS_CUDA_TRY(counted_memcpy(dev.get(), chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice, en.st));
+    L.chunks = dev.get();
+    L.nchunks = (int)chunks.size();
+    return Status::Ok();
+}
+
 Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
 {
     P.ps = ps;
     cudaStream_t st = en.st;
-    int smem_optin = 0;
-    DRESS_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, en.device));
-    const long long smem_cap = smem_optin - 256;
 
     // one launch for all batchable requests
-    int maxE = 1, maxN = 1, maxk = 1, M = 2;
-    long long maxbytes = 16, arena = 0, values = 0, ms_total = 0, nranks = 0;
+    long long arena = 0, values = 0, ms_total = 0, nranks = 0;
     std::vector<ParentDesc> &descs = P.descs;
     std::vector<long long> &val_base = P.val_base;
     // byte / element offsets of each request's sections, turned into device
     // pointers once the buffers exist
     std::vector<long long> data_off, ranks_off, ms_off;
     for (Prep *p : ps) {
-        ParentLayout PL = parent_layout(p->N, p->E, p->S, p->T, 0, 0);
-        maxE = std::max(maxE, p->E);
-        maxN = std::max(maxN, p->N);
-        maxk = std::max(maxk, p->r->k);
-        M = std::max(M, p->M);
-        maxbytes = std::max(maxbytes, PL.bytes);
+        const ImageLayout IL = image_layout(p->N, p->E, p->img.Q, p->img.P2, p->img.uniform, 0, 0);
+        P.maxE = std::max(P.maxE, p->E);
+        P.maxN = std::max(P.maxN, p->N);
+        P.maxk = std::max(P.maxk, p->r->k);
+        P.M = std::max(P.M, p->M);
+        P.max_state = std::max(P.max_state, state_bytes(p->E, p->N, p->r->k, STATE_VALUE));
         ParentDesc d{};
+        d.img = p->img;
         d.N = p->N; d.E = p->E; d.S = p->S; d.T = p->T;
         d.kind = p->r->kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA;
         d.k = p->r->k;
@@ -522,24 +660,15 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
         ms_off.push_back(p->ms_host ? ms_total : -1);
         descs.push_back(d);
         val_base.push_back(values);
-        arena += PL.bytes;
+        arena += IL.bytes;
         values += p->items * (long long)p->E;
         nranks += (long long)p->ranks.size();
         if (p->ms_host) ms_total += p->total * (long long)p->E;
     }
-    Tune tu = pick_tune(maxE, maxN, M, maxk, *en.cfg);
+    bool fits = false;
+    DRESS_TRY(shape_launch(P, en, pick_tune(P.maxE, P.maxN, P.M, P.maxk, *en.cfg), fits));
+    if (!fits) return Status::Err(DRESSX_EUNSUPPORTED, "subgraph state exceeds shared memory");
     BatchLaunch &L = P.L;
-    L.maxE = maxE;
-    L.maxN = maxN;
-    L.maxk = maxk;
-    L.M = M;
-    L.parent_bytes = maxbytes;
-    P.smem_cap = smem_cap;
-    int smem_sm = 0;
-    DRESS_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, en.device));
-    P.smem_sm = smem_sm;
-    if (!shape_launch(L, tu, smem_cap, smem_sm))
-        return Status::Err(DRESSX_EUNSUPPORTED, "subgraph state exceeds shared memory");
 
     // pack parents, several threads for many, into the pinned stage when it
     // can hold them (the upload is then one DMA; the stage is free again
@@ -557,25 +686,12 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
     parallel_for((long long)ps.size(), host_threads((long long)ps.size() / 16), [&](long long ii) {
         const size_t i = (size_t)ii;
         Prep *p = ps[i];
-        p_dress_graph_t g = p->g;
-        ParentLayout PL = parent_layout(p->N, p->E, p->S, p->T, 0, 0);
-        unsigned char *b = hbytes + data_off[i];
-        std::memcpy(b + PL.U, g->U, (size_t)p->E * 4);
-        std::memcpy(b + PL.V, g->V, (size_t)p->E * 4);
-        std::memcpy(b + PL.w, g->edge_weight, (size_t)p->E * 8);
-        std::memcpy(b + PL.row_off, g->adj_offset, (size_t)(p->N + 1) * 4);
-        std::memcpy(b + PL.row_eid, g->adj_edge_idx, (size_t)p->S * 4);
-        std::memcpy(b + PL.ioff, p->ioff.data(), (size_t)(p->E + 1) * 4);
-        if (p->T) std::memcpy(b + PL.pairs, p->pairs.data(), (size_t)p->T * 8);
+        pack_image(p->g, p->ioff, p->pairs, p->img, hbytes + data_off[i]);
         if (!p->ranks.empty()) std::copy(p->ranks.begin(), p->ranks.end(), hranks.begin() + ranks_off[i]);
     }, 16);
-    std::vector<Chunk> &chunks = P.chunks;
-    build_chunks(ps, L.groups, -1, chunks);
-
     const int nreq = (int)ps.size();
     DevBuf<unsigned char> &d_pdata = P.d_pdata;
     DevBuf<ParentDesc> &d_desc = P.d_desc;
-    DevBuf<Chunk> &d_chunks = P.d_chunks;
     DevBuf<long long> &d_ranks = P.d_ranks;
     DevBuf<unsigned long long> &d_vals = P.d_vals, &d_stats = P.d_stats;
     DevBuf<double> &d_ms = P.d_ms;
@@ -584,7 +700,6 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
     P.ms_total = ms_total;
     DRESS_TRY(d_pdata.alloc((size_t)arena, st));
     DRESS_TRY(d_desc.alloc(descs.size(), st));
-    DRESS_TRY(d_chunks.alloc(chunks.size(), st));
     DRESS_TRY(d_ranks.alloc(hranks.size() + 1, st));
     DRESS_TRY(d_vals.alloc((size_t)values + 1, st));
     DRESS_TRY(d_stats.alloc(ST_WORDS * (size_t)nreq, st));
@@ -601,8 +716,7 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
     DRESS_CUDA_TRY(counted_memcpy(d_pdata.get(), hbytes, (size_t)arena, cudaMemcpyHostToDevice, st));
     DRESS_CUDA_TRY(counted_memcpy(d_desc.get(), descs.data(), descs.size() * sizeof(ParentDesc),
                                    cudaMemcpyHostToDevice, st));
-    DRESS_CUDA_TRY(counted_memcpy(d_chunks.get(), chunks.data(), chunks.size() * sizeof(Chunk),
-                                   cudaMemcpyHostToDevice, st));
+    DRESS_TRY(chunk_batch(P, en, P.d_chunks, P.chunks, L));
     if (!hranks.empty())
         DRESS_CUDA_TRY(counted_memcpy(d_ranks.get(), hranks.data(), hranks.size() * sizeof(long long),
                                        cudaMemcpyHostToDevice, st));
@@ -618,10 +732,7 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
             }
     }
     L.parents = d_desc.get();
-    L.chunks = d_chunks.get();
-    L.nchunks = (int)chunks.size();
     L.chunk_counter = d_counter.get();
-    L.per_group = 0;
     P.need_hist = false;
     for (Prep *p : ps) P.need_hist |= p->r->want_histogram != 0;
     if (P.need_hist) DRESS_TRY(P.d_alt.alloc((size_t)values + 1, st));
@@ -737,30 +848,30 @@ Status autotune_batched(BatchPlan &P, const Ctx &en, int *best_out, std::vector<
     int best = -1;
     double best_rate = 0.0;
     Status err;
-    Tune best_tu{0, 0, 1};
+    Tune best_tu{32};
     std::vector<std::pair<double, Tune>> tried;
     for (const Cand &cd : cands) {
-        const int gs = cd.gs;
-        Tune tu{gs, gs == 32 ? 16 : std::min(15, 512 / gs), cd.per_sm};
-        BatchLaunch L = P.L;
-        if (!shape_launch(L, tu, P.smem_cap, P.smem_sm)) {
+        const Tune tu{cd.gs, cd.per_sm};
+        bool fits = false;
+        err = shape_launch(P, en, tu, fits);
+        if (!err.ok()) break;
+        if (!fits || P.per_sm != tu.per_sm) {
             if (rates) rates->push_back(0.f);
             continue;
         }
         // a sample spread over the whole batch: every k-th chunk
         std::vector<Chunk> all, ch;
-        build_chunks(P.ps, L.groups, -1, all);
+        BatchLaunch L = P.L;
+        err = chunk_batch(P, en, d_try, all, L);
+        if (!err.ok()) break;
         const long long k = std::max<long long>(1, (total + limit - 1) / limit);
         for (size_t c = 0; c < all.size(); c += (size_t)k) ch.push_back(all[c]);
         long long items = 0;
         for (const Chunk &c : ch) items += c.count;
-        err = d_try.alloc(ch.size(), st);
-        if (!err.ok()) break;
-        if (cudaMemcpyAsync(d_try.get(), ch.data(), ch.size() * sizeof(Chunk), cudaMemcpyHostToDevice, st) != cudaSuccess) {
+        if (counted_memcpy(d_try.get(), ch.data(), ch.size() * sizeof(Chunk), cudaMemcpyHostToDevice, st) != cudaSuccess) {
             err = Status::Err(DRESSX_ECUDA, "autotune: chunk upload failed");
             break;
         }
-        L.chunks = d_try.get();
         L.nchunks = (int)ch.size();
         float ms = 0.f;
         std::vector<float> times;
@@ -801,17 +912,12 @@ Status autotune_batched(BatchPlan &P, const Ctx &en, int *best_out, std::vector<
     if (best < 0) return Status::Err(DRESSX_EUNSUPPORTED, "autotune: no group size fits");
     {
         std::lock_guard<std::mutex> lk(g_tuned_mu);
-        g_tuned[tune_key(P.L.maxE, P.L.maxN, P.L.M, P.L.maxk)] = best_tu;
+        g_tuned[tune_key(P.maxE, P.maxN, P.M, P.maxk)] = best_tu;
     }
-    if (!shape_launch(P.L, best_tu, P.smem_cap, P.smem_sm))
-        return Status::Err(DRESSX_EUNSUPPORTED, "autotune: re-plan failed");
-    P.tuned_per_sm = best_tu.per_sm;
-    build_chunks(P.ps, P.L.groups, -1, P.chunks);
-    DRESS_TRY(P.d_chunks.alloc(P.chunks.size(), st));
-    DRESS_CUDA_TRY(counted_memcpy(P.d_chunks.get(), P.chunks.data(), P.chunks.size() * sizeof(Chunk),
-                                   cudaMemcpyHostToDevice, st));
-    P.L.chunks = P.d_chunks.get();
-    P.L.nchunks = (int)P.chunks.size();
+    bool fits = false;
+    DRESS_TRY(shape_launch(P, en, best_tu, fits));
+    if (!fits) return Status::Err(DRESSX_EUNSUPPORTED, "autotune: re-plan failed");
+    DRESS_TRY(chunk_batch(P, en, P.d_chunks, P.chunks, P.L));
     if (P.gexec) {                       // the captured stage has the old schedule
         cudaGraphExecDestroy(P.gexec);
         P.gexec = nullptr;
@@ -1249,10 +1355,10 @@ int dressx_batch_autotune(dressx_batch_t *b, int *group_threads, int *ctas_per_s
     Engine &en = engine();
     std::lock_guard<std::mutex> lk(en.mu);
     std::vector<float> r;
-    int best = b->ptrs.empty() ? 0 : b->plan.L.gsize;
+    int best = b->ptrs.empty() ? 0 : b->plan.gsize;
     Status s = b->ptrs.empty() ? Status::Ok() : autotune_batched(b->plan, en.ctx, &best, &r);
     if (group_threads) *group_threads = best;
-    if (ctas_per_sm) *ctas_per_sm = b->plan.tuned_per_sm;
+    if (ctas_per_sm) *ctas_per_sm = b->plan.per_sm;
     if (rates)
         for (int i = 0; i < 8; ++i) rates[i] = i < (int)r.size() ? r[(size_t)i] : 0.f;
     set_last_error(s);

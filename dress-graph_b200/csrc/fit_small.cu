@@ -26,7 +26,6 @@
 namespace dress {
 
 namespace {
-constexpr int SMALL_GSIZE = 512;       // threads of the one group
 // Above about 3000 edges one SM takes longer than the multi-kernel fit over
 // the whole device (measured on G(n, m): 0.21-0.33 ms against 0.95 ms up to
 // 1500 edges, even at 3000, behind beyond).
@@ -155,15 +154,11 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     const long long S = g->adj_offset[N];
     if (g->adj_offset[0] != 0 || S < 0) return Status::Ok();      // fit_graph reports it
 
-    // shape: one group of SMALL_GSIZE threads and the staged parent (the state
-    // and the graph without its pairs must fit before the pairs are found),
-    // else a cluster of 8 CTAs (16 when 8 cannot hold the state)
+    // shape: one CTA that holds the state and the staged graph, else a cluster of 8 CTAs (16 when 8 cannot hold the state)
     int smem_optin = 0;
     DRESS_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
     const long long smem_cap = smem_optin - 1024;
-    bool one_cta = E <= SMALL_MAX_EDGES &&
-                   batch_group_bytes(E, N, 1, SMALL_GSIZE) +
-                           parent_layout(N, E, (int)S, 0, g->NW != nullptr, 1).bytes <= smem_cap;
+    bool one_cta = E <= SMALL_MAX_EDGES && batch_fits(E, N, 0);
     int lnc = -1;
     if (!one_cta) {
         if ((long long)cluster_fit_smem_bytes(E, N, 3) <= smem_cap) lnc = 3;
@@ -192,29 +187,26 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         if (T > INT_MAX / 2) return Status::Ok();
     }
     const int has_nw = g->NW != nullptr;
-    const ParentLayout PL = parent_layout(N, E, (int)S, (int)T, has_nw, 1);
-
     BatchLaunch L{};
-    L.gsize = SMALL_GSIZE;
-    L.groups = 1;
-    L.per_group = 0;
-    L.min_ctas = 1;
-    L.maxE = E;
-    L.maxN = N;
-    L.maxk = 1;
-    L.M = maxdeg + 1;
-    L.parent_bytes = PL.bytes;
-    // On one CTA the graph itself must be staged in shared memory too: read
-    // through L2 by a single SM, the sweeps are latency-bound and the
-    // multi-kernel fit answers sooner (measured on G(2000, 10000): 3.9 ms
-    // against 1.3 ms).
-    L.stage = 1;
-    if (one_cta && (long long)batch_smem_bytes(L) > smem_cap) {
-        one_cta = false;
-        if ((long long)cluster_fit_smem_bytes(E, N, 3) <= smem_cap) lnc = 3;
-        else if ((long long)cluster_fit_smem_bytes(E, N, 4) <= smem_cap) lnc = 4;
-        else return Status::Ok();
+    ImageShape img;
+    if (one_cta) {
+        // On one CTA the graph itself must be staged in shared memory too: read
+        // through L2 by a single SM, the sweeps are latency-bound and the
+        // multi-kernel fit answers sooner (measured on G(2000, 10000): 3.9 ms
+        // against 1.3 ms).
+        img = plan_image(g, ioff, ITEM_PLAIN, 0, has_nw, true);
+        L.ctas = 1;
+        DRESS_TRY(batch_smem(ctx.device, 1, &L.smem));
+        one_cta = chunk_geometry(N, E, 0, img, batch_room(L.smem), BATCH_SM_WARPS, BATCH_SM_WARPS).staged != 0;
+        if (!one_cta) {
+            if ((long long)cluster_fit_smem_bytes(E, N, 3) <= smem_cap) lnc = 3;
+            else if ((long long)cluster_fit_smem_bytes(E, N, 4) <= smem_cap) lnc = 4;
+            else return Status::Ok();
+        }
     }
+    const ParentLayout PL = parent_layout(N, E, (int)S, (int)T, has_nw, 1);
+    const size_t image = one_cta ? (size_t)image_layout(N, E, img.Q, img.P2, img.uniform, img.has_nw, 1).bytes
+                                 : (size_t)PL.bytes;
 
     // One device block holds everything: the packed parent image, the row
     // targets (cluster: the device pair walk reads them), the descriptor, the
@@ -222,7 +214,7 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     // the inputs once, into the context's pinned stage, and one copy each
     // way moves them.
     auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-    const size_t off_tgt = al((size_t)PL.bytes);
+    const size_t off_tgt = al(image);
     const size_t off_desc = al(off_tgt + (one_cta ? 0 : (size_t)S * sizeof(int)));
     const size_t off_chunk = al(off_desc + sizeof(ParentDesc));
     const size_t off_ctr = al(off_chunk + sizeof(Chunk));
@@ -235,19 +227,20 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DRESS_TRY(ctx.stage->reserve(total));
     unsigned char *h = (unsigned char *)ctx.stage->ptr();
     unsigned char *dv = d_blob.get();
-    std::memcpy(h + PL.U, g->U, (size_t)E * 4);
-    std::memcpy(h + PL.V, g->V, (size_t)E * 4);
-    std::memcpy(h + PL.w, g->edge_weight, (size_t)E * 8);
-    std::memcpy(h + PL.row_off, g->adj_offset, (size_t)(N + 1) * 4);
-    if (S) std::memcpy(h + PL.row_eid, g->adj_edge_idx, (size_t)S * 4);
     if (one_cta) {
-        std::memcpy(h + PL.ioff, ioff.data(), (size_t)(E + 1) * 4);
-        if (T) std::memcpy(h + PL.pairs, pairs.data(), (size_t)T * 8);
-    } else if (S) {
-        std::memcpy(h + off_tgt, g->adj_target, (size_t)S * 4);
+        pack_image(g, ioff, pairs, img, h);
+    } else {
+        std::memcpy(h + PL.U, g->U, (size_t)E * 4);
+        std::memcpy(h + PL.V, g->V, (size_t)E * 4);
+        std::memcpy(h + PL.w, g->edge_weight, (size_t)E * 8);
+        std::memcpy(h + PL.row_off, g->adj_offset, (size_t)(N + 1) * 4);
+        if (S) {
+            std::memcpy(h + PL.row_eid, g->adj_edge_idx, (size_t)S * 4);
+            std::memcpy(h + off_tgt, g->adj_target, (size_t)S * 4);
+        }
+        if (has_nw) std::memcpy(h + PL.nw, g->NW, (size_t)N * 8);
+        std::memcpy(h + PL.dinit, g->edge_dress, (size_t)E * 8);
     }
-    if (has_nw) std::memcpy(h + PL.nw, g->NW, (size_t)N * 8);
-    std::memcpy(h + PL.dinit, g->edge_dress, (size_t)E * 8);
     ParentDesc P{};
     P.N = N;
     P.E = E;
@@ -259,14 +252,13 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     P.force_exact = ctx.cfg->exact_sums != 0;
     P.max_iter = max_iterations;
     P.eps = epsilon;
-    P.has_nw = has_nw;
-    P.has_dinit = 1;
+    P.img = img;
     P.data = dv;
     P.values = (double *)(dv + off_vals);
     P.stats = (unsigned long long *)(dv + off_stats);
     P.offset = 0;
     P.stride = 1;
-    const Chunk ch{0, 1, 0};
+    const Chunk ch{0, 1, 0, std::max(1, std::min(BATCH_SM_WARPS, (E + 31) / 32)), 0};
     std::memcpy(h + off_desc, &P, sizeof P);
     std::memcpy(h + off_chunk, &ch, sizeof ch);
     std::memset(h + off_ctr, 0, off_vals - off_ctr);           // counter and statistics
@@ -301,7 +293,7 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     if (one_cta) {
         DRESS_TRY(launch_batch(L, ctx.num_sms, st));
     } else {
-        Status ls = launch_cluster_fit(L.parents, E, N, lnc, ctx.num_sms, st);
+        Status ls = launch_cluster_fit(L.parents, has_nw, E, N, lnc, ctx.num_sms, st);
         if (ls.code == DRESSX_EUNSUPPORTED) return Status::Ok();     // the multi-kernel fit takes it
         DRESS_TRY(ls);
     }

@@ -54,13 +54,6 @@ double ms_between(Clock::time_point a, Clock::time_point b)
     return std::chrono::duration<double, std::milli>(b - a).count();
 }
 
-int next_pow2i(int x)
-{
-    int m = 1;
-    while (m < x) m <<= 1;
-    return m;
-}
-
 // Opt-in shared memory per block of a B200 (used when no device is asked).
 constexpr long long B200_SMEM_OPTIN = 232448;
 // Device bytes per value of a histogram: the values, the sort's second
@@ -70,11 +63,11 @@ constexpr long long HIST_BYTES_PER_VALUE = 56;
 // Pinned staging per lane and finisher at start-up (each grows on demand).
 constexpr size_t STAGE_START_BYTES = (size_t)64 << 20;
 
+// CTAs to an SM in the batch launches, where every state fits its part.
+constexpr int SERVER_CTAS = 2;
+
 // Largest whole-graph fit packed into batch launches.
 constexpr int PLAIN_BATCH_MAX_EDGES = 2048;
-
-// Threads per fit by edge count.
-int gsize_for(int E) { return E <= 640 ? 32 : E <= 2048 ? 64 : E <= 8192 ? 128 : 256; }
 
 int class_of(int kind, int path)
 {
@@ -90,9 +83,9 @@ struct Planned {
     int item_kind = ITEM_PLAIN;
     long long items = 0;                // fits to run on the batch path
     long long num_subgraphs = 0;
-    int N = 0, E = 0, S = 0, T = 0, M = 2, gsize = 32, k = 0;
-    int has_nw = 0, has_dinit = 0, fwd = 0;
-    ParentLayout PL{};
+    int N = 0, E = 0, S = 0, T = 0, k = 0;
+    int fwd = 0;
+    ImageShape img;
     std::vector<unsigned char> packed;  // batch path: the parent image
 };
 
@@ -147,8 +140,7 @@ Status plan_request(p_dress_graph_t g, int kind, int k, long long smem_cap, bool
     // 1 <= k < N (the other orders are trivial or in-place fits, served by
     // the lane path).  A whole-graph fit keeps rows of at most 256
     // neighbours: one thread sums a row there.
-    bool batch = batch_group_bytes(E, N, pl.k, gsize_for(E)) <= smem_cap - 1024 &&
-                 batch_group_bytes(E, N, pl.k, gsize_for(E)) <= BATCH_GROUP_BYTES_MAX;
+    bool batch = batch_fits(E, N, pl.k) && state_bytes(E, N, pl.k, STATE_VALUE) <= batch_room((int)smem_cap);
     if (kind == DRESSX_FIT) batch = batch && maxdeg <= 256;
     if (kind != DRESSX_FIT) batch = batch && k >= 1 && k < N;
     // a whole-graph fit in the batch kernel runs on one thread group (one
@@ -178,36 +170,18 @@ Status plan_request(p_dress_graph_t g, int kind, int k, long long smem_cap, bool
 
     pl.path = DRESSX_PATH_BATCH;
     pl.T = (int)(pairs.size() / 2);
-    pl.M = std::max(2, next_pow2i(maxdeg + 1));
-    pl.gsize = gsize_for(E);
     pl.fwd = g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD;
-    if (kind == DRESSX_FIT) {
-        pl.item_kind = ITEM_PLAIN;
-        pl.items = 1;
-        pl.has_nw = g->NW != nullptr;
-        pl.has_dinit = 1;       // a fit continues from the current edge values
-    } else {
-        pl.item_kind = kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA;
-        pl.items = pl.num_subgraphs;
-    }
-    pl.PL = parent_layout(N, E, S, pl.T, pl.has_nw, pl.has_dinit);
+    pl.item_kind = kind == DRESSX_FIT ? ITEM_PLAIN : kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA;
+    pl.items = kind == DRESSX_FIT ? 1 : pl.num_subgraphs;
+    // a fit continues from the current edge values
+    pl.img = plan_image(g, ioff, pl.item_kind, pl.k, kind == DRESSX_FIT && g->NW, kind == DRESSX_FIT);
+    const ImageLayout IL = image_layout(N, E, pl.img.Q, pl.img.P2, pl.img.uniform, pl.img.has_nw, pl.img.has_dinit);
     const long long out = kind == DRESSX_FIT ? 8LL * (E + N) : 8LL * pl.items * E;
-    pl.bytes = pl.PL.bytes + out + 8LL * ST_WORDS + 4096 +
+    pl.bytes = IL.bytes + out + 8LL * ST_WORDS + 4096 +
                (kind == DRESSX_FIT ? 0 : pl.items * (long long)E * (HIST_BYTES_PER_VALUE - 8));
     if (!pack) return Status::Ok();
-    pl.packed.assign((size_t)pl.PL.bytes, 0);
-    unsigned char *b = pl.packed.data();
-    if (E) {
-        std::memcpy(b + pl.PL.U, g->U, (size_t)E * 4);
-        std::memcpy(b + pl.PL.V, g->V, (size_t)E * 4);
-        std::memcpy(b + pl.PL.w, g->edge_weight, (size_t)E * 8);
-    }
-    std::memcpy(b + pl.PL.row_off, g->adj_offset, (size_t)(N + 1) * 4);
-    if (S) std::memcpy(b + pl.PL.row_eid, g->adj_edge_idx, (size_t)S * 4);
-    std::memcpy(b + pl.PL.ioff, ioff.data(), (size_t)(E + 1) * 4);
-    if (pl.T) std::memcpy(b + pl.PL.pairs, pairs.data(), (size_t)pl.T * 8);
-    if (pl.has_nw) std::memcpy(b + pl.PL.nw, g->NW, (size_t)N * 8);
-    if (pl.has_dinit && E) std::memcpy(b + pl.PL.dinit, g->edge_dress, (size_t)E * 8);
+    pl.packed.assign((size_t)IL.bytes, 0);
+    pack_image(g, ioff, pairs, pl.img, pl.packed.data());
     return Status::Ok();
 }
 
@@ -250,7 +224,8 @@ struct Lane {
 struct Server {
     dressx_server_config_t cfg{};
     int device = 0, sms = 148;
-    long long smem_cap = B200_SMEM_OPTIN - 256;
+    long long smem_cap = B200_SMEM_OPTIN;    // shared memory of a batch CTA: one to an SM,
+    int smem_part = 0;                       // and SERVER_CTAS to an SM
     long long budget = 0;
     cudaMemPool_t pool = nullptr;
     cudaStream_t up = nullptr;            // uploads of admitted batch requests
@@ -323,9 +298,10 @@ Status Server::start(const dressx_server_config_t *c)
     device = cfg.device >= 0 ? cfg.device : en.device;
     DRESS_CUDA_TRY(cudaSetDevice(device));
     DRESS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    int optin = 0;
-    DRESS_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    smem_cap = optin - 256;
+    int full = 0;
+    DRESS_TRY(batch_smem(device, 1, &full));
+    DRESS_TRY(batch_smem(device, SERVER_CTAS, &smem_part));
+    smem_cap = full;
     size_t free_b = 0, total_b = 0;
     DRESS_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     budget = cfg.memory_budget_bytes ? (long long)cfg.memory_budget_bytes
@@ -502,110 +478,57 @@ void Server::credit_locked(Slot *s)
 }
 
 // ---- batch launches ---------------------------------------------------------------
-// Launch geometry for requests of one class: group mode for whole-graph fits,
-// CTA mode (parent staged in shared memory when that leaves enough groups)
-// for subgraph fits.
-bool geometry(BatchLaunch &L, bool plain, long long cap)
-{
-    if (plain) {
-        L.per_group = 1;
-        L.stage = 0;
-        L.groups = std::max(1, 256 / L.gsize);
-        while (L.groups > 1 && (long long)batch_smem_bytes(L) > cap) --L.groups;
-        return (long long)batch_smem_bytes(L) <= cap;
-    }
-    L.per_group = 0;
-    int tg = 512 / L.gsize;
-    if (L.gsize > 32 && tg > 15) tg = 15;
-    L.stage = 1;
-    L.groups = tg;
-    while (L.groups > 1 && (long long)batch_smem_bytes(L) > cap) --L.groups;
-    if ((long long)batch_smem_bytes(L) > cap || L.groups * 2 < tg) {
-        BatchLaunch L2 = L;
-        L2.stage = 0;
-        L2.groups = tg;
-        while (L2.groups > 1 && (long long)batch_smem_bytes(L2) > cap) --L2.groups;
-        if ((long long)batch_smem_bytes(L) > cap || L2.groups > L.groups) L = L2;
-    }
-    return (long long)batch_smem_bytes(L) <= cap;
-}
-
+// A launch holds requests of every kind and size: the kernel divides each
+// CTA's memory by the parent at hand.  Every waiting request gets a slice of a
+// CTA's round per turn until the launch holds launch_work edge-units.
 bool Server::form_launch(Slot *s, BatchLaunch &L, std::vector<ParentDesc> &descs, std::vector<Chunk> &chunks)
 {
-    for (;;) {
-        Req *first = nullptr;
-        for (Req *r : active)
-            if (!r->cancelled && r->err.ok() && r->next_item < r->pl.items) { first = r; break; }
-        if (!first) return false;
-        const bool plain = first->pl.item_kind == ITEM_PLAIN;
-        const int gs = first->pl.gsize;
-        std::vector<Req *> cand;
-        for (Req *r : active)
-            if (!r->cancelled && r->err.ok() && r->next_item < r->pl.items &&
-                (r->pl.item_kind == ITEM_PLAIN) == plain && r->pl.gsize == gs)
-                cand.push_back(r);
-        auto shape = [&](const std::vector<Req *> &rs) {
-            L = BatchLaunch{};
-            L.gsize = gs;
-            L.maxE = 1;
-            L.maxN = 1;
-            L.maxk = 1;
-            L.M = 2;
-            L.parent_bytes = 16;
-            for (Req *r : rs) {
-                L.maxE = std::max(L.maxE, r->pl.E);
-                L.maxN = std::max(L.maxN, r->pl.N);
-                L.maxk = std::max(L.maxk, r->pl.k);
-                L.M = std::max(L.M, r->pl.M);
-                L.parent_bytes = std::max(L.parent_bytes, r->pl.PL.bytes);
-            }
-            return geometry(L, plain, smem_cap);
-        };
-        if (!shape(cand)) {
-            cand.assign(1, first);
-            if (!shape(cand)) {
-                first->err = Status::Err(DRESSX_EUNSUPPORTED, "fit state exceeds shared memory");
-                maybe_finish_locked(this, first);
-                continue;
-            }
+    std::vector<Req *> cand;
+    bool large = false;                      // a state needs more than its part of an SM
+    for (Req *r : active)
+        if (!r->cancelled && r->err.ok() && r->next_item < r->pl.items) {
+            cand.push_back(r);
+            large |= state_bytes(r->pl.E, r->pl.N, r->pl.k, STATE_VALUE) > batch_room(smem_part);
         }
-        // every waiting request of the class gets a slice per round until the
-        // launch holds launch_work edge-units
-        const long long chunk_items = plain ? 1 : L.groups;
-        std::unordered_map<Req *, int> idx;
-        long long work = 0;
-        bool progress = true;
-        while (work < cfg.launch_work && progress) {
-            progress = false;
-            for (Req *r : cand) {
-                if (r->next_item >= r->pl.items) continue;
-                const long long n = std::min(chunk_items, r->pl.items - r->next_item);
-                auto it = idx.find(r);
-                int di;
-                if (it == idx.end()) {
-                    di = (int)descs.size();
-                    idx[r] = di;
-                    descs.push_back(r->desc);
-                    s->credits.push_back({r, 0});
-                    ++r->inflight;
-                    r->started = true;
-                } else {
-                    di = it->second;
-                }
-                chunks.push_back({di, (int)n, r->next_item});
-                r->next_item += n;
-                s->credits[(size_t)di].second += n;
-                work += n * std::max(1, r->pl.E);
-                progress = true;
-                if (work >= cfg.launch_work) break;
-            }
-        }
-        active.erase(std::remove_if(active.begin(), active.end(),
-                                    [](Req *r) { return r->next_item >= r->pl.items; }),
-                     active.end());
-        L.nchunks = (int)chunks.size();
-        return true;
+    if (cand.empty()) return false;
+    L = BatchLaunch{};
+    L.ctas = large ? 1 : SERVER_CTAS;
+    L.smem = large ? (int)smem_cap : smem_part;
+    std::vector<ChunkSource> src;
+    std::vector<long long> slice;
+    for (Req *r : cand) {
+        slice.push_back(chunk_geometry(r->pl.N, r->pl.E, r->pl.k, r->pl.img, batch_room(L.smem),
+                                       BATCH_SM_WARPS / L.ctas, 1).groups);
+        src.push_back({0, r->pl.N, r->pl.E, r->pl.k, r->next_item, 0, r->pl.img});
     }
+    long long work = 0;
+    bool progress = true;
+    while (work < cfg.launch_work && progress) {
+        progress = false;
+        for (size_t i = 0; i < cand.size(); ++i) {
+            Req *r = cand[i];
+            if (r->next_item >= r->pl.items) continue;
+            const long long n = std::min(slice[i], r->pl.items - r->next_item);
+            if (src[i].items == 0) {
+                src[i].parent = (int)descs.size();
+                descs.push_back(r->desc);
+                s->credits.push_back({r, 0});
+                ++r->inflight;
+                r->started = true;
+            }
+            src[i].items += n;
+            s->credits[(size_t)src[i].parent].second += n;
+            r->next_item += n;
+            work += n * std::max(1, r->pl.E);
+            progress = true;
+            if (work >= cfg.launch_work) break;
+        }
+    }
+    active.erase(std::remove_if(active.begin(), active.end(), [](Req *r) { return r->next_item >= r->pl.items; }),
+                 active.end());
+    build_chunks(src, 1, sms, L.ctas, L.smem, chunks);
+    L.nchunks = (int)chunks.size();
+    return true;
 }
 
 Status Server::issue_launch(Slot *s, BatchLaunch &L, const std::vector<ParentDesc> &descs,
@@ -654,8 +577,7 @@ Status Server::admit_batch(Req *r)
     d.fwd = pl.fwd;
     d.max_iter = r->pub->max_iterations;
     d.eps = r->pub->epsilon;
-    d.has_nw = pl.has_nw;
-    d.has_dinit = pl.has_dinit;
+    d.img = pl.img;
     d.data = r->d_data.get();
     d.values = (double *)r->d_values.get();
     d.stats = r->d_stats.get();
@@ -1112,7 +1034,7 @@ int dressx_server_destroy(dressx_server_t *h)
 int dressx_server_estimate(p_dress_graph_t g, int kind, int k, int64_t *bytes, int *path)
 {
     Planned pl;
-    Status s = plan_request(g, kind, k, B200_SMEM_OPTIN - 256, false, pl);
+    Status s = plan_request(g, kind, k, B200_SMEM_OPTIN, false, pl);
     if (!s.ok()) {
         set_last_error(s);
         return s.code;

@@ -120,9 +120,9 @@ int  dressx_batch_create(dressx_hist_request_t *reqs, int n, dressx_batch_t **ou
 /* All fits and histograms on the device; results stay in device memory. */
 int  dressx_batch_run(dressx_batch_t *b);
 /* Autotuner: runs the batch kernel on this batch's subgraphs (a spread
- * sample beyond 200K) with 32, 64, 128 and 256 threads per subgraph and one
- * 512-thread CTA per SM, then 32, 64 and 128 threads with two CTAs sharing
- * each SM -- each schedule where one subgraph's state fits shared memory --
+ * sample beyond 200K) with at least 32, 64, 128 and 256 threads per subgraph
+ * and one 1024-thread CTA per SM, then 32, 64 and 128 threads with two CTAs of
+ * 512 sharing each SM -- where one subgraph's state fits a CTA's memory --
  * timing the median of three runs after an untimed one.  It keeps the first
  * schedule, in that order, within 3 % of the fastest (so schedules closer
  * than the run-to-run noise resolve the same way every time) for the
