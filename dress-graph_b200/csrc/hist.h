@@ -7,15 +7,17 @@
 namespace dress {
 
 // Histogram runs left in device memory: pairs[2r], pairs[2r+1] = (value
-// bits, count) of run r; run_seg[r] = its segment; runs are grouped by
-// segment in segment order.
+// bits, count) of run r, in segment order; segment s has the runs
+// [seg_runs[s], seg_runs[s+1]).
 struct HistResult {
     DevBuf<long long> pairs;
-    DevBuf<int> run_seg;
+    std::vector<long long> seg_runs;
     long long R = 0;
     int nseg = 0;
 };
 
+// keys: the segments' values (raw double bits), overwritten; alt: scratch of
+// the same size, the same indices.
 Status histogram_device(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
                         const std::vector<long long> &len, HistResult &res, cudaStream_t st, int sms);
 Status histogram_download(HistResult &res, std::vector<std::vector<long long>> &out, cudaStream_t st);
@@ -46,8 +48,7 @@ Status segmented_sort(unsigned long long *keys, unsigned long long *alt, const s
 
 // Sorts each segment [begin[s], begin[s]+len[s]) of `keys` (raw double bits)
 // and returns, per segment, the flat [value_bits, count, ...] list ascending
-// by value with ==-equal values merged.  `alt` is scratch of the same size as
-// `keys`; the sorted keys may end up in either buffer.
+// by value.  `alt` is scratch of the same size as `keys`; both are overwritten.
 Status histogram_segments(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
                           const std::vector<long long> &len, std::vector<std::vector<long long>> &out,
                           cudaStream_t st, int sms);

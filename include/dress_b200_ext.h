@@ -157,7 +157,7 @@ int dressx_counters(int64_t *h2d_bytes, int64_t *d2h_bytes, int64_t *launches, i
  * allocate device memory when they need it: code running while a CUDA graph
  * is captured, frameworks whose caching allocator owns the device memory,
  * and loops that must not allocate after start-up.  The call allocates
- * nothing: its scratch is one fixed array of about 16.5 MiB compiled into the
+ * nothing: its scratch is one fixed array of about 16 MiB compiled into the
  * library, which every GPU that loads the library holds until the process
  * exits.
  *   values   device pointer, n doubles (n <= DRESSX_NOALLOC_MAX_VALUES;
