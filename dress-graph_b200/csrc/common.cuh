@@ -135,52 +135,6 @@ struct CSum {
     }
 };
 
-// Compare-exchange putting the smaller value at the lower position.
-__device__ __forceinline__ void cswap(double &a, double &b)
-{
-    bool sw = b < a;
-    double lo = sw ? b : a;
-    double hi = sw ? a : b;
-    a = lo;
-    b = hi;
-}
-
-// Register sorting network on M (power of two) values, ascending.  Bitonic
-// network in its single-direction form: for every block size k the first
-// comparator pairs i with its mirror i^(k-1), the rest pair i with i^j.
-// Missing values are padded with +inf by the caller.
-template <int M>
-__device__ __forceinline__ void sort_regs(double (&a)[M])
-{
-#pragma unroll
-    for (int k = 2; k <= M; k <<= 1) {
-#pragma unroll
-        for (int i = 0; i < M; ++i) {
-            int j = i ^ (k - 1);
-            if (j > i) cswap(a[i], a[j]);
-        }
-#pragma unroll
-        for (int s = k >> 2; s > 0; s >>= 1) {
-#pragma unroll
-            for (int i = 0; i < M; ++i) {
-                int j = i ^ s;
-                if (j > i) cswap(a[i], a[j]);
-            }
-        }
-    }
-}
-
-// Sorted KBN over the first n (1 <= n <= M) register values.
-template <int M>
-__device__ __forceinline__ double kbn_regs(const double (&a)[M], int n)
-{
-    double s = a[0], c = 0.0;
-#pragma unroll
-    for (int i = 1; i < M; ++i)
-        if (i < n) kbn_step(s, c, a[i]);
-    return dadd(s, c);
-}
-
 // Cooperative in-place ascending sort of buf[0..n) by `nthr` threads with
 // index `tid` (a warp or a whole block).  Same single-direction bitonic
 // network over the next power of two; comparators whose upper index is
