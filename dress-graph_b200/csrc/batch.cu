@@ -26,18 +26,13 @@
 // Delta^1 subgraphs of 2,000 regular graphs (16 to 100 vertices): 12.5 ms with
 // a liveness test, a weight and a certificate per term and item, 3.2 ms now;
 // 61 subgraphs of one graph, on one CTA before and one a CTA now: 735 -> 35 us.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <climits>
 #include <map>
 #include <mutex>
-#include <tuple>
 
 #include "batch.h"
 #include "common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace dress {
 namespace {
@@ -123,161 +118,6 @@ __constant__ int c_primes[16] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41,
 __device__ __forceinline__ double marker_weight(int i)
 {
     return dsqrt((double)(i < 16 ? c_primes[i] : 2 * i + 3));
-}
-
-struct View {
-    const int *U, *V, *row_off, *row_eid, *ioff;
-    const double *w, *nw, *dinit;
-    const int2 *pairs;
-};
-
-// ---- a whole graph over a thread-block cluster ---------------------------------
-// Every thread of the cluster is one member of the group; the state arrays are
-// distributed over the CTAs' shared memory, each CTA holding the elements its
-// own threads update in the group loops (element i, visited by group thread
-// i mod size, lives in CTA (i / B) mod n at ((i / (B n)) B + i mod B), B the
-// CTA's threads, n the CTAs).  Other elements are read through distributed
-// shared memory.  sync() is the cluster barrier, which also orders the
-// shared-memory writes of every CTA (no thread spins).
-struct ClusterGroup {
-    int t, size;
-    double *wsl;                 // this CTA's per-warp reduction slots, two parities
-    double *const *part;         // every CTA's two partial slots
-    int ncta;
-    __device__ __forceinline__ void sync() const { cg::this_cluster().sync(); }
-};
-
-struct DArr {
-    double *const *tab;          // every CTA's slice (generic addresses)
-    int lb, lnc;                 // log2 of the CTA's threads and of the CTAs
-    __device__ __forceinline__ double &operator[](int i) const
-    {
-        const int r = (i >> lb) & ((1 << lnc) - 1);
-        const int l = ((i >> (lb + lnc)) << lb) | (i & ((1 << lb) - 1));
-        return tab[r][l];
-    }
-};
-
-template <class Op>
-__device__ __forceinline__ double cluster_reduce(const ClusterGroup &g, double v, int parity, Op op)
-{
-    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int nw = (int)blockDim.x >> 5;
-    if ((threadIdx.x & 31) == 0) g.wsl[parity * nw + (threadIdx.x >> 5)] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = g.wsl[parity * nw];
-        for (int i = 1; i < nw; ++i) m = op(m, g.wsl[parity * nw + i]);
-        g.part[cg::this_cluster().block_rank()][parity] = m;
-    }
-    g.sync();
-    double m = g.part[0][parity];
-    for (int r = 1; r < g.ncta; ++r) m = op(m, g.part[r][parity]);
-    return m;
-}
-
-__device__ __forceinline__ double cluster_max(const ClusterGroup &g, double v, int parity)
-{
-    return fmax(0.0, cluster_reduce(g, v, parity, [](double a, double b) { return fmax(a, b); }));
-}
-
-// Stored terms of vertex u's row, w[e] d[e] of every slot edge
-// (dress.c:566-569).
-struct RowTerms {
-    const int *row_eid;
-    const double *w;
-    DArr d0;
-    int rb;
-    __device__ __forceinline__ bool operator()(int j, double &t) const
-    {
-        const int e = row_eid[rb + j];
-        t = dmul(w[e], d0[e]);
-        return true;
-    }
-};
-
-// Common-neighbour terms of edge (u, v): w[eu] d[eu] + w[ev] d[ev] of every
-// pair (dress.c:485-490)
-struct PairTerms {
-    const int2 *pairs;
-    const double *w;
-    DArr d0;
-    int pb;
-    __device__ __forceinline__ bool operator()(int j, double &t) const
-    {
-        const int2 pr = pairs[pb + j];
-        t = dadd(dmul(w[pr.x], d0[pr.x]), dmul(w[pr.y], d0[pr.y]));
-        return true;
-    }
-};
-
-// The fit of a whole graph by the threads of a cluster.
-__device__ void fit_whole(const ParentDesc &P, const View &G, const ClusterGroup &g, DArr d0, DArr d1, DArr vd)
-{
-    const int N = P.N, E = P.E;
-    for (int e = g.t; e < E; e += g.size) d0[e] = G.dinit ? G.dinit[e] : 1.0;
-    g.sync();
-    int it = 0;
-    double last = 0.0;
-    for (; it < P.max_iter; ++it) {
-        for (int u = g.t; u < N; u += g.size) {
-            const int rb = G.row_off[u], deg = G.row_off[u + 1] - rb;
-            const RowTerms rt{G.row_eid, G.w, d0, rb};
-            vd[u] = dsqrt(item_sum(dmul(4.0, G.nw ? G.nw[u] : 1.0), deg, rt, P.force_exact != 0));
-        }
-        g.sync();
-        double lmax = 0.0;
-        for (int e = g.t; e < E; e += g.size) {
-            const int u = G.U[e], v = G.V[e];
-            const double own = dmul(G.w[e], d0[e]);
-            const double a4u = dmul(4.0, G.nw ? G.nw[u] : 1.0);
-            const double self = P.fwd ? dadd(a4u, own)
-                                      : dadd(dadd(a4u, dmul(4.0, G.nw ? G.nw[v] : 1.0)), dmul(2.0, own));
-            const int pb = G.ioff[e], np = G.ioff[e + 1] - pb;
-            const PairTerms pt{G.pairs, G.w, d0, pb};
-            const double num = item_sum(self, np, pt, P.force_exact != 0);
-            const double den = dmul(vd[u], vd[v]);
-            const double r = den > 0.0 ? ddiv(num, den) : 0.0;
-            d1[e] = r;
-            const double dd = fabs(dsub(d0[e], r));
-            if (dd > lmax) lmax = dd;
-        }
-        // The reduction's barrier already orders this sweep's writes of d1
-        // and its reads of vd and d0 before the next sweep's writes; its
-        // slots alternate by parity.
-        const double m = cluster_max(g, lmax, it & 1);
-        last = m;
-        const DArr t = d0;
-        d0 = d1;
-        d1 = t;
-        if (m < P.eps) break;
-    }
-    const int sweeps = it < P.max_iter ? it + 1 : P.max_iter;
-    for (int e = g.t; e < E; e += g.size) P.values[e] = d0[e];
-    for (int u = g.t; u < N; u += g.size) P.values[E + u] = vd[u];
-    if (g.t == 0) {
-        unsigned long long *st = P.stats;
-        st[ST_SWEEPS] = (unsigned long long)sweeps;
-        st[ST_EDGE_ITERS] = (unsigned long long)E * (unsigned long long)sweeps;
-        st[ST_FITS] = 1ULL;
-        st[ST_ITERATIONS] = (unsigned long long)(it < P.max_iter ? it : P.max_iter);
-        st[ST_DELTA] = (unsigned long long)__double_as_longlong(last);
-    }
-}
-
-__device__ __forceinline__ View view_of(const unsigned char *b, const ParentLayout &PL, int has_nw)
-{
-    View G;
-    G.U = (const int *)(b + PL.U);
-    G.V = (const int *)(b + PL.V);
-    G.w = (const double *)(b + PL.w);
-    G.row_off = (const int *)(b + PL.row_off);
-    G.row_eid = (const int *)(b + PL.row_eid);
-    G.ioff = (const int *)(b + PL.ioff);
-    G.pairs = (const int2 *)(b + PL.pairs);
-    G.nw = has_nw ? (const double *)(b + PL.nw) : nullptr;
-    G.dinit = (const double *)(b + PL.dinit);
-    return G;
 }
 
 // ---- subgraphs in shared memory -------------------------------------------------
@@ -917,120 +757,7 @@ __global__ void __launch_bounds__(32 * BATCH_SM_WARPS, 1) k_batch(BatchLaunch L)
     }
 }
 
-// One whole-graph fit (ParentDesc of kind ITEM_PLAIN) by one cluster of
-// CL_THREADS-thread CTAs.  Shared memory of a CTA: its slices of d, d_next
-// and the vertex norms (per_e, per_e and per_n doubles), the warp slots, its
-// two partials, and the tables of every CTA's slices.
-constexpr int CL_THREADS = 512, CL_LB = 9;
-constexpr int CL_MAX_CTAS = 16;
-
-__global__ void __launch_bounds__(CL_THREADS, 1) k_fit_cluster(const ParentDesc *pp, int has_nw, int per_e, int per_n, int lnc)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    cg::cluster_group cl = cg::this_cluster();
-    const int nc = (int)cl.num_blocks();
-    double *s_d0 = (double *)smem;
-    double *s_d1 = s_d0 + per_e;
-    double *s_vd = s_d1 + per_e;
-    double *wsl = s_vd + per_n;
-    double *part = wsl + 2 * (CL_THREADS / 32);
-    double **tab = (double **)(part + 2);          // [4][CL_MAX_CTAS]: d0, d1, vd, partials
-    if ((int)threadIdx.x < nc) {
-        const unsigned r = threadIdx.x;
-        tab[0 * CL_MAX_CTAS + r] = cl.map_shared_rank(s_d0, r);
-        tab[1 * CL_MAX_CTAS + r] = cl.map_shared_rank(s_d1, r);
-        tab[2 * CL_MAX_CTAS + r] = cl.map_shared_rank(s_vd, r);
-        tab[3 * CL_MAX_CTAS + r] = cl.map_shared_rank(part, r);
-    }
-    cl.sync();                                      // tables ready, every CTA running
-    const ParentDesc P = *pp;
-    const ParentLayout PL = parent_layout(P.N, P.E, P.S, P.T, has_nw, 1);
-    const View G = view_of(P.data, PL, has_nw);
-    const ClusterGroup g{(int)cl.block_rank() * CL_THREADS + (int)threadIdx.x, nc * CL_THREADS, wsl,
-                         (double *const *)(tab + 3 * CL_MAX_CTAS), nc};
-    const DArr d0{tab + 0 * CL_MAX_CTAS, CL_LB, lnc}, d1{tab + 1 * CL_MAX_CTAS, CL_LB, lnc},
-        vd{tab + 2 * CL_MAX_CTAS, CL_LB, lnc};
-    fit_whole(P, G, g, d0, d1, vd);
-    cl.sync();                                      // no CTA leaves while others read its memory
-}
-
-Status launch_cluster_m(const ParentDesc *d_parent, int has_nw, int E, int N, int lnc, int sms, cudaStream_t st)
-{
-    const int nc = 1 << lnc, span = nc * CL_THREADS;
-    const int per_e = ((E + span - 1) / span) * CL_THREADS, per_n = ((N + span - 1) / span) * CL_THREADS;
-    const size_t smem = (size_t)(2 * per_e + per_n + 2 * (CL_THREADS / 32) + 2) * sizeof(double) +
-                        4 * CL_MAX_CTAS * sizeof(double *);
-    // attributes and the placement check are set up once per device and
-    // cluster shape: the queries cost more than a small fit's whole launch
-    int dev = 0;
-    DRESS_CUDA_TRY(cudaGetDevice(&dev));
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, size_t>, int> placeable;      // (device, CTAs, smem) -> clusters
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = placeable.find(std::make_tuple(dev, nc, smem));
-        if (it != placeable.end()) {
-            if (it->second < 1) return Status::Err(DRESSX_EUNSUPPORTED, "cluster fit does not fit the device");
-        }
-    }
-    static std::mutex amu;
-    static std::map<int, size_t> attr_smem;                             // device -> dynamic smem set
-    {
-        std::lock_guard<std::mutex> lk(amu);
-        size_t &have = attr_smem[dev];
-        if (have < smem) {
-            DRESS_CUDA_TRY(cudaFuncSetAttribute(k_fit_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            DRESS_CUDA_TRY(cudaFuncSetAttribute(k_fit_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            have = smem;
-        }
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)nc);
-    cfg.blockDim = dim3(CL_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)nc;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = -1;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = placeable.find(std::make_tuple(dev, nc, smem));
-        if (it != placeable.end()) clusters = it->second;
-    }
-    if (clusters < 0) {
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_fit_cluster, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            clusters = 0;
-        }
-        std::lock_guard<std::mutex> lk(mu);
-        placeable[std::make_tuple(dev, nc, smem)] = clusters;
-    }
-    if (clusters < 1) return Status::Err(DRESSX_EUNSUPPORTED, "cluster fit does not fit the device");
-    count_launch();
-    DRESS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_fit_cluster, d_parent, has_nw, per_e, per_n, lnc));
-    (void)sms;
-    return Status::Ok();
-}
-
 }  // namespace
-
-size_t cluster_fit_smem_bytes(int E, int N, int lnc)
-{
-    const int span = (1 << lnc) * CL_THREADS;
-    const int per_e = ((E + span - 1) / span) * CL_THREADS, per_n = ((N + span - 1) / span) * CL_THREADS;
-    return (size_t)(2 * per_e + per_n + 2 * (CL_THREADS / 32) + 2) * sizeof(double) + 4 * CL_MAX_CTAS * sizeof(double *);
-}
-
-Status launch_cluster_fit(const ParentDesc *d_parent, int has_nw, int E, int N, int lnc, int sms, cudaStream_t st)
-{
-    if (lnc < 0 || (1 << lnc) > CL_MAX_CTAS) return Status::Err(DRESSX_EINVAL, "cluster size out of range");
-    return launch_cluster_m(d_parent, has_nw, E, N, lnc, sms, st);
-}
 
 Status batch_smem(int device, int ctas, int *bytes)
 {

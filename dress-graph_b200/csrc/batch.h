@@ -10,26 +10,26 @@ namespace dress {
 
 enum { ITEM_DELTA = 0, ITEM_NABLA = 1, ITEM_PLAIN = 2 };
 
-// Byte offsets of the packed arrays of a graph for the cluster fit.  Every
-// section of this and of the batch kernel's image starts on a 16-byte
-// boundary, so an image can be staged into shared memory with 16-byte copies.
-struct ParentLayout {
-    long long U, V, w, row_off, row_eid, ioff, pairs, nw, dinit, bytes;
-};
-
+// Packed images are staged into shared memory with 16-byte copies: every
+// section starts on a 16-byte boundary.
 __host__ __device__ inline long long pl_align(long long b) { return (b + 15) & ~15LL; }
 
-__host__ __device__ inline ParentLayout parent_layout(int N, int E, int S, int T, int has_nw, int has_dinit)
+// The graph as the cluster fit reads it: endpoints (u | v << 16), row offsets,
+// slot targets and edge ids (u16), weights (absent when all are one power of
+// two), vertex weights, initial values (absent when all are 1.0).
+struct ClusterLayout {
+    long long uv, off, tgt, eid, w, nw, dinit, bytes;
+};
+
+__host__ __device__ inline ClusterLayout cluster_layout(int N, int E, int S, int uniform, int has_nw, int has_dinit)
 {
-    ParentLayout L;
+    ClusterLayout L;
     long long o = 0;
-    L.U = o;       o = pl_align(o + 4LL * E);
-    L.V = o;       o = pl_align(o + 4LL * E);
-    L.w = o;       o = pl_align(o + 8LL * E);
-    L.row_off = o; o = pl_align(o + 4LL * (N + 1));
-    L.row_eid = o; o = pl_align(o + 4LL * S);
-    L.ioff = o;    o = pl_align(o + 4LL * (E + 1));
-    L.pairs = o;   o = pl_align(o + 8LL * T);
+    L.uv = o;      o = pl_align(o + 4LL * E);
+    L.off = o;     o = pl_align(o + 2LL * (N + 1));
+    L.tgt = o;     o = pl_align(o + 2LL * S);
+    L.eid = o;     o = pl_align(o + 2LL * S);
+    L.w = o;       o = pl_align(o + (uniform ? 0 : 8LL * E));
     L.nw = o;      o = pl_align(o + (has_nw ? 8LL * N : 0));
     L.dinit = o;   o = pl_align(o + (has_dinit ? 8LL * E : 0));
     L.bytes = o;
@@ -97,8 +97,8 @@ struct ParentDesc {
     int fwd;             // FORWARD/BACKWARD self term
     int max_iter;
     double eps;
-    ImageShape img;      // batch kernel: shape of the image at data
-    const unsigned char *data;   // packed arrays (image_layout; the cluster fit: parent_layout)
+    ImageShape img;      // shape of the image at data
+    const unsigned char *data;   // packed arrays (image_layout)
     double *values;      // DELTA/NABLA: live values in completion order;
                          // PLAIN: E final edge values, then N vertex norms
     unsigned long long *stats;   // ST_WORDS counters
@@ -185,11 +185,19 @@ Status launch_batch(const BatchLaunch &L, int sms, cudaStream_t st);
 // that it leaves for images and states.
 Status batch_smem(int device, int ctas, int *bytes);
 __host__ __device__ inline long long batch_room(int smem) { return smem - BATCH_HEADER; }
-// One whole-graph fit (the ITEM_PLAIN descriptor at d_parent) by one cluster
-// of 2^lnc CTAs whose shared memory holds the state (cluster_fit_smem_bytes
-// per CTA).  DRESSX_EUNSUPPORTED when such a cluster cannot be placed.
-Status launch_cluster_fit(const ParentDesc *d_parent, int has_nw, int E, int N, int lnc, int sms, cudaStream_t st);
-size_t cluster_fit_smem_bytes(int E, int N, int lnc);
+// One whole-graph fit by one cluster (fit_cluster.cu).  img: Q = the row slots.
+struct ClusterFit {
+    int N, E, fwd, max_iter;
+    double eps;
+    ImageShape img;
+    const unsigned char *data;           // cluster_layout
+    unsigned *pairs, *cursor;            // room for sum_e min(deg u, deg v) words; zero
+    double *values;                      // E final edge values, then N vertex norms
+    unsigned long long *stats;           // ST_FITS 0: a product left the range, nothing was fitted
+};
+// Whether one CTA's memory holds the values and norms.
+bool cluster_fits(int E, int N, int S);
+Status launch_cluster_fit(const ClusterFit &f, cudaStream_t st);
 // A graph is batchable when one subgraph's smallest state fits.
 constexpr long long BATCH_STATE_MAX = 227 * 1024 - BATCH_HEADER;
 inline bool batch_fits(int E, int N, int k)
@@ -210,6 +218,9 @@ void merge_walk_pairs(p_dress_graph_t g, std::vector<int> &ioff, std::vector<int
 ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind, int k, bool has_nw, bool has_dinit);
 void pack_image(p_dress_graph_t g, const std::vector<int> &ioff, const std::vector<int> &pairs, const ImageShape &s,
                 unsigned char *dst);
+// The same for the cluster fit (max_deg: the longest row).
+ImageShape plan_cluster(p_dress_graph_t g, int max_deg);
+void pack_cluster(p_dress_graph_t g, const ImageShape &s, unsigned char *dst);
 // Chunks of a launch: parent p's items, divided so that every SM has work
 // (limit >= 0: only the first `limit` items of the whole batch).
 struct ChunkSource {

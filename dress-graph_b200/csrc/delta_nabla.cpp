@@ -133,13 +133,19 @@ namespace {
 // below 8), PLO about 2^-41 n^2: only products of zero or of values far from
 // any fixed point are outside.  All in units of the weight where that is one
 // power of two.  span = 0: no fast path.
-void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageShape &s)
+// w_max > 0: for the cluster fit, whose sums take terms of any size in any
+// order: PHI then only has to be above the products that occur.  Values stay
+// below about 2 sqrt(nw_max / nw_min); PHI is 16 to 32 times the largest weight
+// times that root, and PLO follows from it.
+void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageShape &s, double w_max = 0.0)
 {
     s.lo = s.span = 0;
     const double unit = s.uniform ? s.wc : 1.0;
     const double A = 4.0 * nw_min / unit, Amax = 4.0 * nw_max / unit;
     if (!(A >= 0x1p-300) || !(Amax <= 0x1p300)) return;
-    const double phi = std::ldexp(1.0, std::ilogb(A) + (fwd ? 0 : 1));
+    if (!(w_max <= 0x1p300)) return;
+    double phi = std::ldexp(1.0, std::ilogb(A) + (fwd ? 0 : 1));
+    if (w_max > 0.0) phi = std::max(4.0 * phi, std::ldexp(1.0, std::ilogb(16.0 * w_max / unit * std::sqrt(Amax / A)) + 1));
     const double n = most_terms;
     const double bound = 2.0 * Amax + 2.0 * (n + 1.0) * phi;
     const double plo = std::ldexp(1.0, std::ilogb(n * bound * 0x1p-50) + 1);
@@ -149,6 +155,38 @@ void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageSha
     std::memcpy(&b1, &phi, 8);
     s.lo = (unsigned)(b0 >> 32);
     s.span = (unsigned)(b1 >> 32) - s.lo;
+}
+
+}  // namespace
+
+namespace {
+
+// every weight the same power of two
+void uniform_weight(p_dress_graph_t g, ImageShape &s)
+{
+    const int E = g->E;
+    s.wc = 1.0;
+    s.uniform = 1;
+    if (E == 0) return;
+    int ex = 0;
+    const double w0 = g->edge_weight[0];
+    bool same = w0 > 0.0 && std::isfinite(w0) && std::frexp(w0, &ex) == 0.5 && std::abs(ex) <= 300;
+    for (int e = 1; e < E && same; ++e) same = g->edge_weight[e] == w0;
+    s.uniform = same;
+    if (same) s.wc = w0;
+}
+
+// smallest and largest vertex weight (lo NaN where one is)
+void weight_bounds(p_dress_graph_t g, double &lo, double &hi)
+{
+    lo = hi = 1.0;
+    if (!g->NW || g->N == 0) return;
+    lo = hi = g->NW[0];
+    for (int u = 1; u < g->N && !std::isnan(lo); ++u) {
+        const double x = g->NW[u];
+        if (x < lo || std::isnan(x)) lo = x;
+        if (x > hi) hi = x;
+    }
 }
 
 }  // namespace
@@ -170,31 +208,47 @@ ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind,
         s.P2 += p;
         most = std::max(most, 2 * p + 1);
     }
-    s.wc = 1.0;
-    if (E > 0) {
-        int ex = 0;
-        const double w0 = g->edge_weight[0];
-        bool same = w0 > 0.0 && std::isfinite(w0) && std::frexp(w0, &ex) == 0.5 && std::abs(ex) <= 300;
-        for (int e = 1; e < E && same; ++e) same = g->edge_weight[e] == w0;
-        s.uniform = same;
-        if (same) s.wc = w0;
-    } else {
-        s.uniform = 1;
-    }
+    uniform_weight(g, s);
     double lo = 1.0, hi = 1.0;
-    if (kind == ITEM_PLAIN && has_nw && N > 0) {
-        lo = hi = g->NW[0];
-        for (int u = 1; u < N; ++u) {
-            lo = g->NW[u] < lo ? g->NW[u] : lo;
-            hi = g->NW[u] > hi ? g->NW[u] : hi;
-            if (std::isnan(g->NW[u])) lo = g->NW[u];
-            if (std::isnan(lo)) break;
-        }
-    } else if (kind == ITEM_NABLA && k > 0) {
-        hi = std::sqrt((double)std::max(53, 2 * k + 1));      // no marker weight is larger
-    }
+    if (kind == ITEM_PLAIN && has_nw) weight_bounds(g, lo, hi);
+    else if (kind == ITEM_NABLA && k > 0) hi = std::sqrt((double)std::max(53, 2 * k + 1));   // no marker is larger
     fast_range(lo, hi, most, g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD, s);
     return s;
+}
+
+ImageShape plan_cluster(p_dress_graph_t g, int max_deg)
+{
+    ImageShape s;
+    const int E = g->E;
+    s.Q = g->adj_offset[g->N];
+    uniform_weight(g, s);
+    double lo, hi, w_max = 0.0;
+    weight_bounds(g, lo, hi);
+    s.has_nw = g->NW && !(lo == 1.0 && hi == 1.0);
+    for (int e = 0; e < E; ++e) {
+        s.has_dinit |= g->edge_dress[e] != 1.0;
+        w_max = g->edge_weight[e] > w_max ? g->edge_weight[e] : w_max;
+    }
+    // a row's or an edge's terms, and the merges of its partial sums
+    if (w_max > 0.0)
+        fast_range(lo, hi, max_deg + 16, g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD, s,
+                   w_max);
+    return s;
+}
+
+void pack_cluster(p_dress_graph_t g, const ImageShape &s, unsigned char *dst)
+{
+    const int N = g->N, E = g->E;
+    const ClusterLayout L = cluster_layout(N, E, s.Q, s.uniform, s.has_nw, s.has_dinit);
+    unsigned *uv = (unsigned *)(dst + L.uv);
+    uint16_t *off = (uint16_t *)(dst + L.off), *tgt = (uint16_t *)(dst + L.tgt), *eid = (uint16_t *)(dst + L.eid);
+    for (int e = 0; e < E; ++e) uv[e] = (unsigned)g->U[e] | (unsigned)g->V[e] << 16;
+    for (int u = 0; u <= N; ++u) off[u] = (uint16_t)g->adj_offset[u];
+    for (int q = 0; q < s.Q; ++q) tgt[q] = (uint16_t)g->adj_target[q];
+    for (int q = 0; q < s.Q; ++q) eid[q] = (uint16_t)g->adj_edge_idx[q];
+    if (!s.uniform) std::memcpy(dst + L.w, g->edge_weight, (size_t)E * 8);
+    if (s.has_nw) std::memcpy(dst + L.nw, g->NW, (size_t)N * 8);
+    if (s.has_dinit) std::memcpy(dst + L.dinit, g->edge_dress, (size_t)E * 8);
 }
 
 void pack_image(p_dress_graph_t g, const std::vector<int> &ioff, const std::vector<int> &pairs, const ImageShape &s,

@@ -1,0 +1,75 @@
+"""The one-launch cluster fit at the sizes and values where it changes shape,
+bit for bit against the oracle: one and two value buffers, one to eight lanes a
+vertex, edges a thread owns one to four of, variants, vertex weights, values to
+go on from, and weights that take the fit off this path."""
+import numpy as np
+import pytest
+
+import dress_b200 as db
+from dress_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def _fit(oracle_port, n, U, V, W=None, NW=None, variant=db.UNDIRECTED, one_launch=True, **kw):
+    ref = oracle_port.fit(n, U, V, W, NW, variant=variant, **kw)
+    with db.Graph(n, U, V, W, NW, variant) as g:
+        db.counters(reset=True)
+        it, delta = db.fit_graph(g, kw.get("max_iterations", 100), kw.get("epsilon", 1e-6))
+        launches = db.counters()["launches"]
+        assert one_launch is None or (launches == 1) == one_launch
+        assert (it, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+        np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
+
+
+@pytest.mark.parametrize("n,m", [(700, 2049), (2000, 8191), (2000, 8193), (2000, 10000), (120, 4000), (2600, 13000),
+                                 (2700, 13300), (9000, 16385), (4000, 20000), (3600, 24576), (400, 24001),
+                                 (8000, 22000), (16000, 24575), (500, 1025), (60000, 1500)])
+def test_sizes(n, m, oracle_port):
+    n, U, V = graphs.erdos_renyi(n, m, seed=m)
+    rng = np.random.default_rng(m)
+    W = rng.uniform(0.5, 2.0, m) if m % 2 else None
+    _fit(oracle_port, n, U, V, W)
+
+
+@pytest.mark.parametrize("variant", [db.UNDIRECTED, db.DIRECTED, db.FORWARD, db.BACKWARD])
+@pytest.mark.parametrize("weights", ["none", "third", "wide"])
+def test_variants_and_weights(variant, weights, oracle_port):
+    n, U, V = graphs.erdos_renyi(900, 5003, seed=7)
+    rng = np.random.default_rng(variant)
+    W = {"none": None, "third": np.full(5003, 0.3), "wide": np.exp(rng.uniform(-6, 6, 5003))}[weights]
+    NW = rng.uniform(0.3, 5.0, n) if weights != "none" else None
+    # products over 37 binades and growing (FORWARD, BACKWARD) leave the range
+    _fit(oracle_port, n, U, V, W, NW, variant, one_launch=None if weights == "wide" else True)
+
+
+def test_multigraph_and_isolated_parts(oracle_port):
+    """Parallel edges, self loops, isolated vertices and edges."""
+    rng = np.random.default_rng(3)
+    U = rng.integers(0, 800, 4000).astype(np.int32)
+    V = rng.integers(0, 800, 4000).astype(np.int32)
+    U[:50], V[:50] = np.arange(1000, 1050), np.arange(1050, 1100)
+    _fit(oracle_port, 1200, U, V)
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 3, 7])
+def test_few_sweeps_and_going_on(iterations, oracle_port):
+    n, U, V = graphs.erdos_renyi(1000, 6000, seed=9)
+    _fit(oracle_port, n, U, V, max_iterations=iterations)
+    _fit(oracle_port, n, U, V, max_iterations=iterations, epsilon=0.0)
+    # a second call goes on from the first one's values
+    full = oracle_port.fit(n, U, V)
+    with db.Graph(n, U, V) as g:
+        db.fit_graph(g, iterations, 0.0)
+        it, delta = db.fit_graph(g, 100, 1e-6)
+        assert it + iterations == full["iterations"] and delta == full["delta"]
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), full["edge_dress"].view(np.int64))
+
+
+@pytest.mark.parametrize("bad", [0.0, -0.001, 1e-300, np.inf])
+def test_a_weight_out_of_range_goes_the_other_way(bad, oracle_port):
+    n, U, V = graphs.erdos_renyi(600, 3000, seed=11)
+    W = np.random.default_rng(1).uniform(0.5, 2.0, 3000)
+    W[1234] = bad
+    _fit(oracle_port, n, U, V, W, one_launch=False)
