@@ -218,6 +218,8 @@ void merge_walk_pairs(p_dress_graph_t g, std::vector<int> &ioff, std::vector<int
 ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind, int k, bool has_nw, bool has_dinit);
 void pack_image(p_dress_graph_t g, const std::vector<int> &ioff, const std::vector<int> &pairs, const ImageShape &s,
                 unsigned char *dst);
+// The range of products (lo, span) for sums of up to `most` terms in any order.
+ImageShape plan_products(double nw_min, double nw_max, long long most, bool fwd, double w_max);
 // The same for the cluster fit (max_deg: the longest row).
 ImageShape plan_cluster(p_dress_graph_t g, int max_deg);
 void pack_cluster(p_dress_graph_t g, const ImageShape &s, unsigned char *dst);

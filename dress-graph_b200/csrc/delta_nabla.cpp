@@ -216,6 +216,13 @@ ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind,
     return s;
 }
 
+ImageShape plan_products(double nw_min, double nw_max, long long most, bool fwd, double w_max)
+{
+    ImageShape s;                            // products in full: uniform stays 0
+    if (w_max > 0.0) fast_range(nw_min, nw_max, (int)std::min<long long>(most, 1 << 30), fwd, s, w_max);
+    return s;
+}
+
 ImageShape plan_cluster(p_dress_graph_t g, int max_deg)
 {
     ImageShape s;

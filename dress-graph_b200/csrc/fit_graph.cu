@@ -31,6 +31,7 @@
 #include <thread>
 #include <vector>
 
+#include "batch.h"
 #include "common.cuh"
 #include "engine.h"
 #include "hist.h"
@@ -55,7 +56,9 @@ __device__ __forceinline__ unsigned lanemask_lt()
 // ------------------------------------------------------------------------
 
 // flags[0]: malformed input, flags[1]: a row repeats a neighbour,
-// flags[2]: edge weights are not all bit-identical, flags[3]: max row length.
+// flags[2]: edge weights are not all bit-identical, flags[3]: max row length,
+// flags[4..5]: the largest positive weight (bits of the double), flags[8..11]:
+// the smallest and largest vertex weight (k_nw_bounds).
 // One warp per row (a hub's row is spread over the lanes).  A row outside
 // [0, S) or with end < begin is flagged and not read, so a malformed
 // adj_offset never leads to a read outside adj_target.
@@ -96,10 +99,38 @@ __global__ void k_validate_rows(int N, int E, long long S, const int *off, const
 __global__ void k_validate_edges(int N, int E, const int *U, const int *V, const double *w, int *flags)
 {
     unsigned long long w0 = E > 0 ? (unsigned long long)__double_as_longlong(w[0]) : 0ULL;
+    double wm = 0.0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
         int u = U[e], v = V[e];
         if (u < 0 || u >= N || v < 0 || v >= N) atomicOr(&flags[0], 8);
-        if ((unsigned long long)__double_as_longlong(w[e]) != w0) flags[2] = 1;
+        const double we = w[e];
+        if ((unsigned long long)__double_as_longlong(we) != w0) flags[2] = 1;
+        wm = we > wm ? we : wm;
+    }
+    for (int o = 16; o > 0; o >>= 1) wm = fmax(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    if ((threadIdx.x & 31) == 0 && wm > 0.0)
+        atomicMax((unsigned long long *)(flags + 4), (unsigned long long)__double_as_longlong(wm));
+}
+
+// Smallest and largest vertex weight as bits of positive doubles; a weight that
+// is not positive (or NaN) makes the smallest 0.
+__global__ void k_nw_bounds(int N, const double *nw, unsigned long long *lohi)
+{
+    unsigned long long lo = ~0ULL, hi = 0ULL;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        const double x = nw[i];
+        const unsigned long long b = x > 0.0 ? (unsigned long long)__double_as_longlong(x) : 0ULL;
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long l = __shfl_xor_sync(0xffffffffu, lo, o), h = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = l < lo ? l : lo;
+        hi = h > hi ? h : hi;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (lo < *(volatile unsigned long long *)&lohi[0]) atomicMin(&lohi[0], lo);
+        if (hi > *(volatile unsigned long long *)&lohi[1]) atomicMax(&lohi[1], hi);
     }
 }
 
@@ -744,14 +775,15 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // ---- validate the rows ---------------------------------------------------
     DevBuf<int> d_flags, d_deg, d_cnt;
-    DRESS_TRY(d_flags.alloc(8, st));
+    DRESS_TRY(d_flags.alloc(12, st));
     DRESS_TRY(d_deg.alloc((size_t)N, st));
     DRESS_TRY(d_cnt.alloc((size_t)E, st));
-    DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get(), 0, 8 * sizeof(int), st));
+    DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get(), 0, 12 * sizeof(int), st));
+    DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get() + 8, 0xff, 2 * sizeof(int), st));
     count_launch(), k_validate_rows<<<grid_for((long long)N * 32, 256, 16 * sms), 256, 0, st>>>(
         N, E, S, d_off.get(), d_tgt.get(), d_eidx.get(), d_deg.get(), d_flags.get());
     DRESS_CUDA_TRY(cudaGetLastError());
-    int flags[8];
+    int flags[12];
     DRESS_CUDA_TRY(counted_memcpy(flags, d_flags.get(), sizeof(flags), cudaMemcpyDeviceToHost, st));
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));
     double t_valid = ms_since(t0) - t_upload;
@@ -762,17 +794,26 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     // The edge arrays, validated once they are on the device: before the
     // pairs unless the triangle listing (CSR only) makes them.
     bool uniform = true;
+    double w_max = 0.0, nw_lo = 1.0, nw_hi = 1.0;      // NULL vertex weights mean all 1.0
     auto validate_edges = [&]() -> Status {
         DRESS_TRY(edge_up.join());
         const auto v0 = std::chrono::steady_clock::now();
         count_launch(), k_validate_edges<<<grid_for(E, 256, 16 * sms), 256, 0, st>>>(N, E, d_U.get(), d_V.get(),
                                                                                       d_w.get(), d_flags.get());
+        if (g->NW && N)
+            count_launch(), k_nw_bounds<<<grid_for(N, 256, 16 * sms), 256, 0, st>>>(
+                N, d_nw.get(), (unsigned long long *)(d_flags.get() + 8));
         DRESS_CUDA_TRY(cudaGetLastError());
         DRESS_CUDA_TRY(counted_memcpy(flags, d_flags.get(), sizeof(flags), cudaMemcpyDeviceToHost, st));
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
         t_valid += ms_since(v0);
         if (flags[0]) return Status::Err(DRESSX_EINVAL, "malformed graph (CSR or edge endpoints out of range)");
         uniform = flags[2] == 0;
+        std::memcpy(&w_max, flags + 4, sizeof w_max);
+        if (g->NW && N) {
+            std::memcpy(&nw_lo, flags + 8, sizeof nw_lo);
+            std::memcpy(&nw_hi, flags + 10, sizeof nw_hi);
+        }
         return Status::Ok();
     };
     const bool tri_path = !(g->precompute_intercepts && g->intercept_offset) &&
@@ -1112,6 +1153,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DevBuf<unsigned long long> d_maxd;
     DRESS_TRY(d_vd.alloc((size_t)(N > 0 ? N : 1), st));
     DRESS_TRY(d_maxd.alloc(RING, st));
+    const bool unit_nw = nw_lo == 1.0 && nw_hi == 1.0;
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));
     double setup_ms = ms_since(t0);
     cudaEvent_t sw0, sw1;
@@ -1126,9 +1168,6 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     s.eu = d_eu.get(); s.ev = d_ev.get();
     s.w = uniform ? nullptr : d_wi.get();
     s.wc = wc;
-    bool unit_nw = true;                       // NULL vertex weights mean all 1.0
-    if (g->NW)
-        for (int i = 0; i < N && unit_nw; ++i) unit_nw = g->NW[i] == 1.0;
     s.nw = unit_nw ? nullptr : d_nwi.get();
     s.ioff = d_ioff.get(); s.pairs = d_pairs.get();
     s.vd = d_vd.get(); s.maxd = d_maxd.get();
@@ -1155,20 +1194,43 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DRESS_CUDA_TRY(cudaMemsetAsync(d_maxd.get(), 0, RING * sizeof(unsigned long long), st));
     s.iter = d_iter.get();
     s.max_iter = max_iterations;
+    // the range of products in which sums need no certificate, for this
+    // graph's longest row (no edge has more pairs)
+    DevBuf<int> d_cert;
+    DRESS_TRY(d_cert.alloc(1, st));
+    {
+        const int never = INT_MAX;
+        DRESS_CUDA_TRY(counted_memcpy(d_cert.get(), &never, sizeof(int), cudaMemcpyHostToDevice, st));
+    }
+    s.cert_from = d_cert.get();
+    const ImageShape range = plan_products(nw_lo, nw_hi, max_row + 64, fwd != 0, w_max);
+    s.lo = range.lo;
+    s.span = range.span;
+    bool fast = range.span != 0 && !s.force_exact;
+    const Tiles vtiles = vertex_tiles(vb), etiles = edge_tiles(ec);
     Sweep sw2[2] = {s, s};
     for (int par = 0; par < 2; ++par) {
         sw2[par].d = dbuf[par]; sw2[par].dn = dbuf[par ^ 1];
         sw2[par].p = pbuf[par]; sw2[par].pn = pbuf[par ^ 1];
     }
-    auto enqueue_pair = [&]() -> Status {
-        for (int par = 0; par < 2; ++par) {
-            if (uniform) DRESS_TRY(launch_sweep<true>(sw2[par], vb, ec, lc));
-            else         DRESS_TRY(launch_sweep<false>(sw2[par], vb, ec, lc));
-            count_launch(), k_next_sweep<<<1, 1, 0, st>>>(d_iter.get(), d_maxd.get());
-            DRESS_CUDA_TRY(cudaGetLastError());
-        }
+    auto enqueue = [&](int par) -> Status {
+        if (fast && uniform) DRESS_TRY(launch_fast_sweep<true>(sw2[par], vtiles, etiles, lc));
+        else if (fast)       DRESS_TRY(launch_fast_sweep<false>(sw2[par], vtiles, etiles, lc));
+        else if (uniform)    DRESS_TRY(launch_sweep<true>(sw2[par], vb, ec, lc));
+        else                 DRESS_TRY(launch_sweep<false>(sw2[par], vb, ec, lc));
+        count_launch(), k_next_sweep<<<1, 1, 0, st>>>(d_iter.get(), d_maxd.get(), d_qcount.get(),
+                                                      fast ? d_cert.get() : nullptr);
+        DRESS_CUDA_TRY(cudaGetLastError());
         return Status::Ok();
     };
+    auto enqueue_pair = [&]() -> Status {
+        DRESS_TRY(enqueue(0));
+        return enqueue(1);
+    };
+    if (fast) {
+        if (uniform) count_launch(), k_fast_start<true><<<eg, 256, 0, st>>>(sw2[0]);
+        else         count_launch(), k_fast_start<false><<<eg, 256, 0, st>>>(sw2[0]);
+    }
     cudaGraphExec_t gexec = nullptr;
     long long pair_launches = 0;
     {
@@ -1198,17 +1260,26 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     double last_delta = 0.0;
     while (done < max_iterations && conv < 0) {
         for (int r = 0; r < chunk / 2; ++r) {
-            if (gexec) {
+            if (gexec && !(done & 1)) {
                 count_launch((int)pair_launches);
                 DRESS_CUDA_TRY(cudaGraphLaunch(gexec, st));
             } else {
-                DRESS_TRY(enqueue_pair());
+                DRESS_TRY(enqueue(done & 1));
+                DRESS_TRY(enqueue(~done & 1));
             }
         }
-        const int hi = done + chunk < max_iterations ? done + chunk : max_iterations;
+        int hi = done + chunk < max_iterations ? done + chunk : max_iterations;
         DRESS_CUDA_TRY(counted_memcpy(hmax, d_maxd.get(), RING * sizeof(unsigned long long),
                                        cudaMemcpyDeviceToHost, st));
+        int cert = INT_MAX;
+        if (fast) DRESS_CUDA_TRY(counted_memcpy(&cert, d_cert.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
+        if (cert < hi) {                  // the sweeps from `cert` on did not run
+            hi = std::max(cert, done);
+            fast = false;
+            if (gexec) cudaGraphExecDestroy(gexec);
+            gexec = guard.g = nullptr;
+        }
         for (int it = done; it < hi; ++it) {
             double m;
             std::memcpy(&m, &hmax[it % RING], sizeof(m));
@@ -1222,7 +1293,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         // cost their launches (≈ 3 µs each), a short chunk costs one more
         // host round trip.
         int next = chunk < MAX_CHUNK ? 2 * chunk : MAX_CHUNK;
-        if (conv < 0 && done >= 4) {
+        if (conv < 0 && done >= 4 && cert == INT_MAX) {
             double m1, m0;
             std::memcpy(&m1, &hmax[(done - 1) % RING], sizeof(m1));
             std::memcpy(&m0, &hmax[(done - 4) % RING], sizeof(m0));

@@ -1,0 +1,84 @@
+"""The multi-kernel fit's fast sweeps, bit for bit against the oracle: every
+class of rows and edges (a thread, 8, 16, 32 lanes, a block), and fits that
+leave the fast range at the start, in the middle, or never."""
+import numpy as np
+import pytest
+
+import dress_b200 as db
+from dress_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def multi_kernel():
+    db.configure(one_launch_max_edges=-1)
+    yield
+    db.configure()
+
+
+def _fit(oracle_port, n, U, V, W=None, NW=None, variant=db.UNDIRECTED, **kw):
+    ref = oracle_port.fit(n, U, V, W, NW, variant=variant, **kw)
+    with db.Graph(n, U, V, W, NW, variant) as g:
+        it, delta = db.fit_graph(g, kw.get("max_iterations", 100), kw.get("epsilon", 1e-6))
+        assert (it, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+        np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
+
+
+def _dense_core(rng):
+    """A core of 1,100 vertices joined at random (rows of 500 to 700, as many
+    common neighbours as pairs of a thread to a block take), two hubs over all
+    of 6,000 vertices, and sparse rest."""
+    core = np.argwhere(np.triu(rng.random((700, 700)) < 0.4, 1))
+    thin = np.argwhere(np.triu(rng.random((400, 400)) < 0.08, 1)) + 700
+    hubs = [(6000 + h, x) for h in range(2) for x in range(6000)] + [(6000, 6001)]
+    rest = rng.integers(1100, 6000, (8000, 2))
+    e = np.concatenate([core, thin, np.array(hubs), rest])
+    e = np.sort(e[e[:, 0] != e[:, 1]], axis=1)
+    e = np.unique(e, axis=0)
+    e = e[rng.permutation(len(e))].astype(np.int32)
+    return 6002, e[:, 0].copy(), e[:, 1].copy()
+
+
+@pytest.mark.parametrize("weights", ["none", "uniform", "third"])
+def test_every_class(weights, oracle_port):
+    rng = np.random.default_rng(1)
+    n, U, V = _dense_core(rng)
+    m = len(U)
+    W = {"none": None, "uniform": rng.uniform(0.5, 2.0, m), "third": np.full(m, 0.3)}[weights]
+    NW = rng.uniform(0.5, 2.0, n) if weights == "uniform" else None
+    _fit(oracle_port, n, U, V, W, NW)
+
+
+@pytest.mark.parametrize("m", [1, 2, 255, 256, 257, 5000, 30001])
+def test_sizes(m, oracle_port):
+    n, U, V = graphs.erdos_renyi(max(3, m // 3), m, seed=m)
+    _fit(oracle_port, n, U, V, np.random.default_rng(m).uniform(0.5, 2.0, m))
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 5, 9, 33])
+def test_sweep_limits(iterations, oracle_port):
+    n, U, V = graphs.chung_lu(900, 6000, 2.3, 400, seed=3)
+    _fit(oracle_port, n, U, V, max_iterations=iterations, epsilon=0.0)
+
+
+@pytest.mark.parametrize("bad", [0.0, -0.001, 1e-300])
+def test_out_of_range_from_the_start(bad, oracle_port):
+    n, U, V = graphs.chung_lu(900, 6000, 2.3, 400, seed=3)
+    W = np.random.default_rng(2).uniform(0.5, 2.0, 6000)
+    W[::7] = bad
+    _fit(oracle_port, n, U, V, W)
+
+
+@pytest.mark.parametrize("variant", [db.FORWARD, db.BACKWARD])
+@pytest.mark.parametrize("spread", [4.0, 5.0, 6.0, 7.0, 8.0])
+@pytest.mark.parametrize("iterations", [9, 100])
+def test_out_of_range_on_the_way(variant, spread, iterations, oracle_port):
+    """Directed rows with weights over many binades grow for dozens of sweeps;
+    the certified sweeps take over at an even or an odd one."""
+    n, U, V = graphs.erdos_renyi(900, 5003, seed=7)
+    rng = np.random.default_rng(int(spread * 10))
+    W = np.exp(rng.uniform(-spread, spread, 5003))
+    NW = rng.uniform(0.3, 5.0, n)
+    _fit(oracle_port, n, U, V, W, NW, variant, max_iterations=iterations)
