@@ -848,11 +848,7 @@ Status exec_batched(BatchPlan &P, const Ctx &en)
 }
 
 // Results of the last run into the requests' host-side state.
-// pre/cap (nullable): host arrays already allocated per request, with
-// their capacity in int64 words; the histograms that fit go there (their
-// ownership passes to the request, the entry is cleared).
-Status collect_batched(BatchPlan &P, const Ctx &en, std::vector<int64_t *> *pre = nullptr,
-                       const std::vector<long long> *cap = nullptr)
+Status collect_batched(BatchPlan &P, const Ctx &en)
 {
     cudaStream_t st = en.st;
     const int nreq = (int)P.ps.size();
@@ -866,7 +862,7 @@ Status collect_batched(BatchPlan &P, const Ctx &en, std::vector<int64_t *> *pre 
     if (P.need_hist) {
         std::vector<int64_t *> outs;
         std::vector<long long> lens;
-        DRESS_TRY(histogram_fetch(P.hist, outs, lens, en.stage, st, en.num_sms, pre, cap));
+        DRESS_TRY(histogram_fetch(P.hist, outs, lens, en.stage, st));
         for (int i = 0; i < nreq; ++i) {
             std::free(ps[(size_t)i]->hist_mal);
             ps[(size_t)i]->hist_mal = outs[(size_t)i];
@@ -1014,66 +1010,12 @@ Status capture_batched(BatchPlan &P, const Ctx &en)
     return Status::Ok();
 }
 
-// Host arrays for the histograms, allocated while the fits run.  A request's
-// histogram has at most one pair per value, and it has at most subgraphs x
-// edges values, so arrays of that size are allocated and their pages mapped
-// (a write to each page) by host threads during the device work; the fetch
-// then only copies, and trims each array to its length.  Only when the
-// bounds add up to a moderate size.
-constexpr long long PREFAULT_MIN_BYTES = 64LL << 20;
-constexpr long long PREFAULT_MAX_BYTES = 4LL << 30;
-
-struct Prefault {
-    std::vector<int64_t *> arr;
-    std::vector<long long> cap;          // int64 words
-    std::vector<std::thread> th;
-    void start(const std::vector<Prep *> &ps)
-    {
-        long long total = 0;
-        cap.assign(ps.size(), 0);
-        for (size_t i = 0; i < ps.size(); ++i)
-            if (ps[i]->r->want_histogram) {
-                cap[i] = 2 * ps[i]->items * (long long)ps[i]->E;
-                total += cap[i] * 8;
-            }
-        arr.assign(ps.size(), nullptr);
-        if (total < PREFAULT_MIN_BYTES || total > PREFAULT_MAX_BYTES) return;
-        // leave a core to the thread that drives the device
-        const int nthr = std::max(1, host_threads((long long)ps.size()) - 1);
-        for (int t = 0; t < nthr; ++t)
-            th.emplace_back([this, t, nthr] {
-                for (size_t i = (size_t)t; i < cap.size(); i += (size_t)nthr) {
-                    if (!cap[i]) continue;
-                    const size_t n = (size_t)cap[i] * sizeof(int64_t);
-                    char *a = (char *)std::malloc(n);
-                    if (a)
-                        for (size_t o = 0; o < n; o += 4096) ((volatile char *)a)[o] = 0;
-                    arr[i] = (int64_t *)a;
-                }
-            });
-    }
-    void join()
-    {
-        for (auto &t : th) t.join();
-        th.clear();
-    }
-    ~Prefault()
-    {
-        join();
-        for (int64_t *a : arr) std::free(a);
-    }
-};
-
 Status run_batched(std::vector<Prep *> &ps, const Ctx &en)
 {
     BatchPlan P;
     DRESS_TRY(plan_batched(ps, en, P));
-    Prefault pf;
-    pf.start(ps);
-    Status s = exec_batched(P, en);
-    pf.join();
-    DRESS_TRY(s);
-    return collect_batched(P, en, pf.arr.empty() ? nullptr : &pf.arr, &pf.cap);
+    DRESS_TRY(exec_batched(P, en));
+    return collect_batched(P, en);
 }
 
 Status finish(Prep &p)

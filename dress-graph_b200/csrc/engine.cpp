@@ -131,13 +131,13 @@ void for_pieces(const HostSpan *spans, int n, size_t lo, size_t hi, F fn)
 
 // host copy of chunk k between its stage slot and the spans, split over
 // host threads in 2 MiB grains
-void host_part(const HostSpan *spans, int n, char *stage, size_t k, size_t total, bool to_stage)
+void host_part(const HostSpan *spans, int n, char *stage, size_t k, size_t total, bool to_stage, int threads)
 {
     constexpr size_t grain = (size_t)2 << 20;
     char *slot = stage + (k & 1) * STAGE_CHUNK;
     const size_t lo = k * STAGE_CHUNK, hi = std::min(total, lo + STAGE_CHUNK);
     const long long pieces = (long long)((hi - lo + grain - 1) / grain);
-    parallel_for(pieces, host_threads(pieces), [&](long long g) {
+    parallel_for(pieces, std::min(threads, host_threads(pieces)), [&](long long g) {
         const size_t a = lo + (size_t)g * grain, b = std::min(hi, a + grain);
         for_pieces(spans, n, a, b, [&](const HostSpan &sp, size_t off, size_t len, size_t at) {
             char *st = slot + (a - lo) + at;
@@ -147,7 +147,7 @@ void host_part(const HostSpan *spans, int n, char *stage, size_t k, size_t total
     });
 }
 
-Status staged_copy(const HostSpan *spans, int n, Pinned *pin, cudaStream_t cs, bool up)
+Status staged_copy(const HostSpan *spans, int n, Pinned *pin, cudaStream_t cs, bool up, int threads = 16)
 {
     size_t total = 0;
     for (int i = 0; i < n; ++i) total += spans[i].bytes;
@@ -181,7 +181,7 @@ Status staged_copy(const HostSpan *spans, int n, Pinned *pin, cudaStream_t cs, b
         char *slot = stage + (k & 1) * STAGE_CHUNK;
         const size_t lo = k * STAGE_CHUNK, hi = std::min(total, lo + STAGE_CHUNK);
         if (k >= 2) DRESS_CUDA_TRY(cudaEventSynchronize(ev[k & 1]));     // the slot's last copy is done
-        if (up) host_part(spans, n, stage, k, total, true);
+        if (up) host_part(spans, n, stage, k, total, true, threads);
         Status err;
         for_pieces(spans, n, lo, hi, [&](const HostSpan &sp, size_t off, size_t len, size_t at) {
             cudaError_t e = up ? cudaMemcpyAsync((char *)sp.dev + off, slot + at, len, cudaMemcpyHostToDevice, cs)
@@ -196,29 +196,29 @@ Status staged_copy(const HostSpan *spans, int n, Pinned *pin, cudaStream_t cs, b
         if (!up && k >= 1) {
             // the previous chunk is on the host: copy it out while this one is in flight
             DRESS_CUDA_TRY(cudaEventSynchronize(ev[(k - 1) & 1]));
-            host_part(spans, n, stage, k - 1, total, false);
+            host_part(spans, n, stage, k - 1, total, false, threads);
         }
     }
     if (!up) {
         DRESS_CUDA_TRY(cudaEventSynchronize(ev[(nchunks - 1) & 1]));
-        host_part(spans, n, stage, nchunks - 1, total, false);
+        host_part(spans, n, stage, nchunks - 1, total, false, threads);
     }
     return Status::Ok();
 }
 
 }  // namespace
 
-Status staged_upload(const HostSpan *spans, int n, const Ctx &ctx)
+Status staged_upload(const HostSpan *spans, int n, const Ctx &ctx, int threads)
 {
-    return staged_copy(spans, n, ctx.stage, ctx.st, true);
+    return staged_copy(spans, n, ctx.stage, ctx.st, true, threads);
 }
-Status staged_download(const HostSpan *spans, int n, const Ctx &ctx)
+Status staged_download(const HostSpan *spans, int n, const Ctx &ctx, int threads)
 {
-    return staged_copy(spans, n, ctx.stage, ctx.st, false);
+    return staged_copy(spans, n, ctx.stage, ctx.st, false, threads);
 }
-Status staged_upload_via(const HostSpan *spans, int n, Pinned *stage, cudaStream_t st)
+Status staged_upload_via(const HostSpan *spans, int n, Pinned *stage, cudaStream_t st, int threads)
 {
-    return staged_copy(spans, n, stage, st, true);
+    return staged_copy(spans, n, stage, st, true, threads);
 }
 
 thread_local cudaMemPool_t tls_pool = nullptr;

@@ -165,11 +165,11 @@ constexpr size_t STAGE_CHUNK = (size_t)32 << 20;
 // without being read first, which takes a third of the memory traffic off a
 // large copy between pageable memory and a pinned stage.
 void copy_nt(void *dst, const void *src, size_t n);
-Status staged_upload(const HostSpan *spans, int n, const Ctx &ctx);
-Status staged_download(const HostSpan *spans, int n, const Ctx &ctx);
+Status staged_upload(const HostSpan *spans, int n, const Ctx &ctx, int threads = 16);
+Status staged_download(const HostSpan *spans, int n, const Ctx &ctx, int threads = 16);
 // the same upload through a given stage, on a given stream (the caller's
 // thread must have the stream's device current)
-Status staged_upload_via(const HostSpan *spans, int n, Pinned *stage, cudaStream_t st);
+Status staged_upload_via(const HostSpan *spans, int n, Pinned *stage, cudaStream_t st, int threads = 16);
 
 // ---- device utilities (scan.cu) -------------------------------------------
 // out[i] = sum_{j<i} in[i] for i in [0, n], out[n] = total.  `tmp` must hold

@@ -40,6 +40,7 @@
 namespace dress {
 namespace {
 
+constexpr long long INLINE_COPY_BYTES = 16LL << 20;    // graphs copied by the caller's thread
 constexpr int MAX_CHUNK = 32;      // sweeps launched per host check (<= RING/2)
 constexpr int LOCALITY_MIN_EDGES = 1 << 20;   // graphs renumbered for gather locality
 using namespace sweep;
@@ -670,11 +671,16 @@ struct BackgroundUpload {
     Status result;
     bool running = false;
     double wait_ms = 0.0;                  // time the caller spent blocked in join()
-    Status start(std::vector<HostSpan> spans, const Ctx &ctx)
+    // inline_copy: on the caller's thread after all
+    Status start(std::vector<HostSpan> spans, const Ctx &ctx, bool inline_copy)
     {
         // the destination buffers were allocated in stream order on ctx.st
         DRESS_CUDA_TRY(cudaEventRecord(ctx.fork, ctx.st));
         DRESS_CUDA_TRY(cudaStreamWaitEvent(ctx.side2, ctx.fork, 0));
+        if (inline_copy) {
+            result = staged_upload_via(spans.data(), (int)spans.size(), ctx.stage2, ctx.side2, 1);
+            return result;
+        }
         try {
             th = std::thread([this, sp = std::move(spans), &ctx]() {
                 const cudaError_t e = cudaSetDevice(ctx.device);
@@ -744,6 +750,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // ---- upload: the CSR first; the edge arrays on a host thread of their
     // own, beside the row validation and the triangle listing (CSR only) --------
+    const int few = 8.0 * (double)S + 24.0 * E + 12.0 * N <= (double)INLINE_COPY_BYTES ? 1 : 16;
     DevBuf<int> d_off, d_tgt, d_eidx, d_U, d_V;
     DevBuf<double> d_w, d_d, d_nw;
     DRESS_TRY(d_off.alloc((size_t)N + 1, st));
@@ -755,10 +762,12 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DRESS_TRY(d_d.alloc((size_t)E, st));
     DRESS_TRY(d_nw.alloc((size_t)N, st));
     {
+        // (a graph of few bytes on this thread alone: helper threads that must
+        // first be scheduled cost more than they copy)
         const HostSpan csr[3] = {{g->adj_offset, d_off.get(), ((size_t)N + 1) * sizeof(int)},
                                  {g->adj_target, d_tgt.get(), (size_t)S * sizeof(int)},
                                  {g->adj_edge_idx, d_eidx.get(), (size_t)S * sizeof(int)}};
-        DRESS_TRY(staged_upload(csr, 3, ctx));
+        DRESS_TRY(staged_upload(csr, 3, ctx, few));
     }
     BackgroundUpload edge_up;
     {
@@ -767,7 +776,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
                                        {g->edge_weight, d_w.get(), (size_t)E * sizeof(double)},
                                        {g->edge_dress, d_d.get(), (size_t)E * sizeof(double)}};
         if (g->NW) spans.push_back({g->NW, d_nw.get(), (size_t)N * sizeof(double)});
-        DRESS_TRY(edge_up.start(std::move(spans), ctx));
+        DRESS_TRY(edge_up.start(std::move(spans), ctx, few == 1));
     }
     const double t_upload = ms_since(t0);
     if (!g->NW && N)                           // NULL vertex weights mean all 1.0
@@ -1323,7 +1332,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     {
         const HostSpan spans[2] = {{g->edge_dress, d_out.get(), (size_t)E * sizeof(double)},
                                    {g->vertex_dress, d_out.get() + E, (size_t)N * sizeof(double)}};
-        DRESS_TRY(staged_download(spans, 2, ctx));
+        DRESS_TRY(staged_download(spans, 2, ctx, few));
     }
     if (iterations) *iterations = conv >= 0 ? conv : max_iterations;
     if (delta) *delta = last_delta;

@@ -1071,15 +1071,13 @@ Status histogram_device(unsigned long long *keys, unsigned long long *alt, const
 }
 
 Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vector<long long> &lens, Pinned *stage,
-                       cudaStream_t st, int sms, std::vector<int64_t *> *pre, const std::vector<long long> *cap,
-                       int max_threads)
+                       cudaStream_t st, int max_threads)
 {
     const int nseg = res.nseg;
     outs.assign((size_t)nseg, nullptr);
     lens.assign((size_t)nseg, 0);
     const long long R = res.R;
     if (R == 0) return Status::Ok();
-    (void)sms;
     std::vector<long long> first((size_t)nseg, 0);
     for (int sg = 0; sg < nseg; ++sg) {
         first[(size_t)sg] = res.seg_runs[(size_t)sg];
@@ -1101,9 +1099,10 @@ Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vecto
     // a barrier (a segment may reach into later parts) maps the pages of its
     // part's share of the arrays while the downloads stream in -- the page
     // faults of fresh memory cost more than the copy -- then copies its
-    // share once its part landed.  A final barrier precedes the trimming of
-    // given arrays to their length.
-    const int nthr = pinned && bytes > (64u << 20) ? std::min(max_threads, host_threads((long long)(bytes >> 23))) : 1;
+    // share once its part landed.  From 4 MiB on a thread per MiB: 14 MB took
+    // one thread 4.3 ms.  Below, the caller's thread does it all and waits by
+    // spinning: an event's blocking wait costs 0.3 ms.
+    const int nthr = pinned && bytes > (4u << 20) ? std::min(max_threads, host_threads((long long)(bytes >> 20))) : 1;
     const int parts = std::max(1, nthr);
     std::vector<long long> pcut((size_t)parts + 1);
     for (int t = 0; t <= parts; ++t) pcut[(size_t)t] = R * t / parts;
@@ -1112,14 +1111,15 @@ Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vecto
     for (int t = 0; t < parts && err.ok(); ++t) {
         const long long r0 = pcut[(size_t)t], r1 = pcut[(size_t)t + 1];
         if (r1 <= r0) continue;
-        if (cudaEventCreateWithFlags(&ev[(size_t)t], cudaEventDisableTiming | cudaEventBlockingSync) != cudaSuccess) {
+        if (parts > 1 &&
+            cudaEventCreateWithFlags(&ev[(size_t)t], cudaEventDisableTiming | cudaEventBlockingSync) != cudaSuccess) {
             ev[(size_t)t] = nullptr;
             err = Status::Err(DRESSX_ECUDA, "event creation failed");
             break;
         }
         cudaError_t e = counted_memcpy(host + 2 * r0, res.pairs.get() + 2 * r0, 2 * (size_t)(r1 - r0) * sizeof(long long),
                                        cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaEventRecord(ev[(size_t)t], st);
+        if (e == cudaSuccess && parts > 1) e = cudaEventRecord(ev[(size_t)t], st);
         if (e != cudaSuccess) err = Status::Err(DRESSX_ECUDA, std::string("histogram download: ") + cudaGetErrorString(e));
     }
     // segments in part order: the first segment whose runs reach into each part
@@ -1132,16 +1132,15 @@ Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vecto
             seg0[(size_t)t] = sg;
         }
     }
-    std::vector<char> given((size_t)nseg, 0);    // segments that took a given array
     std::atomic<bool> nomem{false};
     std::mutex mu;
     std::condition_variable cv;
     int ready = 0;                               // parts landed; -1 once the downloads failed
-    int arrived[2] = {0, 0};                     // barrier counts
-    auto barrier = [&](int b) {
+    int arrived = 0;                             // parts whose arrays are allocated
+    auto barrier = [&] {
         std::unique_lock<std::mutex> lk(mu);
-        if (++arrived[b] == parts) cv.notify_all();
-        else cv.wait(lk, [&] { return arrived[b] == parts; });
+        if (++arrived == parts) cv.notify_all();
+        else cv.wait(lk, [&] { return arrived == parts; });
     };
     auto part_work = [&](int t) {
         const long long p0 = pcut[(size_t)t], p1 = pcut[(size_t)t + 1];
@@ -1149,32 +1148,28 @@ Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vecto
         for (int sg = seg0[(size_t)t]; sg < nseg && first[(size_t)sg] < p1; ++sg) {
             const size_t n = (size_t)lens[(size_t)sg] * sizeof(int64_t);
             if (!n || first[(size_t)sg] < p0) continue;
-            if (pre && (*pre)[(size_t)sg] && lens[(size_t)sg] <= (*cap)[(size_t)sg]) {
-                outs[(size_t)sg] = (*pre)[(size_t)sg];
-                (*pre)[(size_t)sg] = nullptr;
-                given[(size_t)sg] = 1;
-                continue;
-            }
             outs[(size_t)sg] = (int64_t *)std::malloc(n);
             if (!outs[(size_t)sg]) nomem = true;
         }
-        barrier(0);
+        barrier();
         // this part's share of segment sg: runs [a, b)
         auto share = [&](int sg, long long &a, long long &b) {
             a = std::max(p0, first[(size_t)sg]);
             b = std::min(p1, first[(size_t)sg] + lens[(size_t)sg] / 2);
         };
-        if (parts > 1)
-            for (int sg = seg0[(size_t)t]; sg < nseg && first[(size_t)sg] < p1; ++sg) {
-                long long a, b;
-                share(sg, a, b);
-                char *o = (char *)outs[(size_t)sg];
-                if (b <= a || !o || given[(size_t)sg]) continue;
-                const size_t lo_b = (size_t)(a - first[(size_t)sg]) * 16, hi_b = (size_t)(b - first[(size_t)sg]) * 16;
-                for (size_t x = lo_b; x < hi_b; x += 4096) ((volatile char *)o)[x] = 0;
-            }
+        for (int sg = seg0[(size_t)t]; sg < nseg && first[(size_t)sg] < p1; ++sg) {
+            long long a, b;
+            share(sg, a, b);
+            char *o = (char *)outs[(size_t)sg];
+            if (b <= a || !o) continue;
+            const size_t lo_b = (size_t)(a - first[(size_t)sg]) * 16, hi_b = (size_t)(b - first[(size_t)sg]) * 16;
+            for (size_t x = lo_b; x < hi_b; x += 4096) ((volatile char *)o)[x] = 0;
+        }
         bool ok;
-        {
+        if (parts == 1) {
+            ok = err.ok() && cudaStreamSynchronize(st) == cudaSuccess;
+            if (!ok && err.ok()) err = Status::Err(DRESSX_ECUDA, "histogram download failed");
+        } else {
             std::unique_lock<std::mutex> lk(mu);
             cv.wait(lk, [&] { return ready < 0 || ready > t; });
             ok = ready > t;
@@ -1185,21 +1180,16 @@ Status histogram_fetch(HistResult &res, std::vector<int64_t *> &outs, std::vecto
                 share(sg, a, b);
                 int64_t *o = outs[(size_t)sg];
                 if (b <= a || !o) continue;
-                copy_nt(o + 2 * (a - first[(size_t)sg]), host + 2 * a, (size_t)(b - a) * 16);
-            }
-        barrier(1);
-        // trim the given arrays of the segments starting here (shrinking keeps the data)
-        for (int sg = seg0[(size_t)t]; sg < nseg && first[(size_t)sg] < p1; ++sg)
-            if (given[(size_t)sg] && first[(size_t)sg] >= p0 && lens[(size_t)sg] < (*cap)[(size_t)sg]) {
-                void *r2 = std::realloc(outs[(size_t)sg], (size_t)lens[(size_t)sg] * sizeof(int64_t));
-                if (r2) outs[(size_t)sg] = (int64_t *)r2;
+                // (a small result stays in the cache for its reader)
+                if (parts == 1) std::memcpy(o + 2 * (a - first[(size_t)sg]), host + 2 * a, (size_t)(b - a) * 16);
+                else copy_nt(o + 2 * (a - first[(size_t)sg]), host + 2 * a, (size_t)(b - a) * 16);
             }
     };
     std::vector<std::thread> th;
     if (parts > 1)
         for (int t = 0; t < parts; ++t) th.emplace_back(part_work, t);
     // this thread waits for the downloads in order and releases the parts
-    for (int t = 0; t < parts && err.ok(); ++t) {
+    for (int t = 0; parts > 1 && t < parts && err.ok(); ++t) {
         if (ev[(size_t)t] && cudaEventSynchronize(ev[(size_t)t]) != cudaSuccess) {
             err = Status::Err(DRESSX_ECUDA, "histogram download failed");
         } else {

@@ -711,7 +711,7 @@ Status collect_batch(Server *sv, Req *r, Ctx *ctx)
     std::vector<int64_t *> outs;
     std::vector<long long> lens;
     // at most 8 copy threads: lanes and other finishers share the host
-    DRESS_TRY(histogram_fetch(res, outs, lens, ctx->stage, ctx->st, sv->sms, nullptr, nullptr, 8));
+    DRESS_TRY(histogram_fetch(res, outs, lens, ctx->stage, ctx->st, 8));
     p->hist_flat = outs[0];
     p->hist_len = (int)lens[0];
     return Status::Ok();
