@@ -1194,14 +1194,13 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     double *dbuf[2] = {d_dbuf.get(), d_dbuf.get() + E};
     double *pbuf[2] = {uniform ? nullptr : d_pbuf.get(), uniform ? nullptr : d_pbuf.get() + E};
 
-    // Two sweeps (the even one writes buffer 1, the odd one buffer 0) and the
-    // index steps between them are captured once into a CUDA graph, replayed
-    // for every pair of sweeps; the host reads the ring after each chunk.
+    // An even sweep writes buffer 1, an odd one buffer 0; the device keeps the
+    // sweep's index and the host reads the ring of maxima after each chunk.
     DevBuf<int> d_iter;
-    DRESS_TRY(d_iter.alloc(1, st));
-    DRESS_CUDA_TRY(cudaMemsetAsync(d_iter.get(), 0, sizeof(int), st));
+    DRESS_TRY(d_iter.alloc(2, st));
+    DRESS_CUDA_TRY(cudaMemsetAsync(d_iter.get(), 0, 2 * sizeof(int), st));
     DRESS_CUDA_TRY(cudaMemsetAsync(d_maxd.get(), 0, RING * sizeof(unsigned long long), st));
-    s.iter = d_iter.get();
+    s.iter = s.next = d_iter.get();
     s.max_iter = max_iterations;
     // the range of products in which sums need no certificate, for this
     // graph's longest row (no edge has more pairs)
@@ -1223,12 +1222,11 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         sw2[par].p = pbuf[par]; sw2[par].pn = pbuf[par ^ 1];
     }
     auto enqueue = [&](int par) -> Status {
-        if (fast && uniform) DRESS_TRY(launch_fast_sweep<true>(sw2[par], vtiles, etiles, lc));
-        else if (fast)       DRESS_TRY(launch_fast_sweep<false>(sw2[par], vtiles, etiles, lc));
-        else if (uniform)    DRESS_TRY(launch_sweep<true>(sw2[par], vb, ec, lc));
-        else                 DRESS_TRY(launch_sweep<false>(sw2[par], vb, ec, lc));
-        count_launch(), k_next_sweep<<<1, 1, 0, st>>>(d_iter.get(), d_maxd.get(), d_qcount.get(),
-                                                      fast ? d_cert.get() : nullptr);
+        if (fast && uniform) return launch_fast_sweep<true>(sw2[par], vtiles, etiles, lc);
+        if (fast) return launch_fast_sweep<false>(sw2[par], vtiles, etiles, lc);
+        if (uniform) DRESS_TRY(launch_sweep<true>(sw2[par], vb, ec, lc));
+        else         DRESS_TRY(launch_sweep<false>(sw2[par], vb, ec, lc));
+        count_launch(), k_next_sweep<<<1, 1, 0, st>>>(d_iter.get(), d_maxd.get(), d_qcount.get());
         DRESS_CUDA_TRY(cudaGetLastError());
         return Status::Ok();
     };
@@ -1240,9 +1238,13 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         if (uniform) count_launch(), k_fast_start<true><<<eg, 256, 0, st>>>(sw2[0]);
         else         count_launch(), k_fast_start<false><<<eg, 256, 0, st>>>(sw2[0]);
     }
+    // A pair of certified sweeps (up to 36 launches) and its index steps is
+    // captured once into a CUDA graph and replayed.  A fast sweep is two
+    // launches: capturing and instantiating them (0.4 ms) costs more than the
+    // replays save.
     cudaGraphExec_t gexec = nullptr;
     long long pair_launches = 0;
-    {
+    if (!fast) {
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
         const long long before = tls_launches;
         cudaGraph_t graph = nullptr;
@@ -1286,8 +1288,6 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         if (cert < hi) {                  // the sweeps from `cert` on did not run
             hi = std::max(cert, done);
             fast = false;
-            if (gexec) cudaGraphExecDestroy(gexec);
-            gexec = guard.g = nullptr;
         }
         for (int it = done; it < hi; ++it) {
             double m;

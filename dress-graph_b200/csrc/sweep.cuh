@@ -83,6 +83,7 @@ struct Sweep {
     int exact_cap;                 // terms an exact-sort block holds in shared memory
     int force_exact;               // queue every item (tests of the exact path)
     int *cert_from;                // first sweep whose products are not all in the fast range
+    int *next;                     // the same word as iter, and the blocks done behind it
     unsigned lo, span;             // that range (high words)
 };
 
@@ -100,13 +101,12 @@ __device__ __forceinline__ bool skipped(const Sweep &s)
 
 __device__ __forceinline__ unsigned long long *max_slot(const Sweep &s) { return &s.maxd[*s.iter % RING]; }
 
-// end of a sweep: the next index, its slot and the exact queues cleared.
-// cert_from (fast sweeps; else null): a sweep that did not run is not counted.
-__global__ void k_next_sweep(int *iter, unsigned long long *maxd, unsigned *qcount, const int *cert_from)
+// end of a certified sweep: the next index, its slot and the exact queues
+// cleared (a fast sweep's last block does its own)
+__global__ void k_next_sweep(int *iter, unsigned long long *maxd, unsigned *qcount)
 {
     qcount[0] = 0u;
     qcount[1] = 0u;
-    if (cert_from && *iter >= *cert_from) return;
     const int it = *iter + 1;
     *iter = it;
     maxd[it % RING] = 0ULL;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(EXACT_THR) k_edge_exact(Sweep s)
 // A phase is one launch: every item class is cut into tiles, the heaviest class
 // first, and one wave of blocks takes the tiles in turn, so no class waits for
 // the tail of another.  On a 200,003-edge power-law graph the sixteen launches
-// of a sweep took 105 us of 2 to 20 us kernels; three take 22 us.  28 M edges on
+// of a sweep took 105 us of 2 to 20 us kernels; two take 22 us.  28 M edges on
 // one box: 1.41 -> 1.19 ms a weighted sweep, 1.33 -> 1.09 ms unweighted (1.29 and
 // 1.21 ms with 7 or 8 resident blocks, which spill).
 // Rows and edges of more than MED_CAP terms take a block each: a warp's 128
@@ -722,6 +722,17 @@ __global__ void __launch_bounds__(FAST_THR, FAST_RESIDENT) k_edge_fast(Sweep s, 
     }
     if (out) atomicMin(s.cert_from, *s.iter + 1);
     block_max_to(max_slot(s), lmax);
+    // the last block ends the sweep: the next index, its slot cleared
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&s.next[1], 1) == (int)gridDim.x - 1) {
+            s.next[1] = 0;
+            const int it = s.next[0] + 1;
+            s.maxd[it % RING] = 0ULL;
+            s.next[0] = it;
+        }
+    }
 }
 
 // cert_from of the initial products (INT_MAX: all in range)
