@@ -10,18 +10,17 @@
 //     lowest-rank vertex); other variants and multigraphs from the
 //     reference's exact merge walk per edge; graphs built with
 //     precompute_intercepts reuse their own tables.
-//   * vertices and edges are renumbered so that items with the same number of
-//     sum terms are contiguous ("bins": 1, 2, 4, 8, 16, 32 terms -> one thread
-//     per item with a register sorting network; <=1024 -> one warp per item
-//     with a shared-memory sort; more -> one block per item).  Renumbering
-//     makes every per-edge stream (endpoints, weight, value, next value)
-//     sequential and packs the edges that appear in triangles -- the only ones
-//     gathered by the edge sweep -- into one L2-sized region at the end.
+//   * vertices are renumbered so that rows of one size class are contiguous, and
+//     the edges without common neighbours come first; the rest is listed by
+//     size class.  A large graph's edges are ordered by owner for the locality
+//     of the sweeps' gathers, a smaller one's by size class.  Every per-edge
+//     stream (endpoints, weight, value, next value) is sequential.
 //   * p = w*d is stored next to d (double-buffered) for weighted graphs, so a
 //     term costs one gather; for uniform weights p is formed on the fly.
-// Each sweep is one vertex-norm pass and one edge pass per bin; the edge pass
-// folds max|d_next - d| into a per-sweep slot, and every kernel of sweep i
-// returns at once if sweep i-1 already met the tolerance, so a chunk of
+// A sweep is one vertex-norm launch and one edge launch while all products stay
+// in the fast range, else certified launches per size class (sweep.cuh).  The
+// edge pass folds max|d_next - d| into a per-sweep slot, and every kernel of
+// sweep i returns at once if sweep i-1 already met the tolerance, so a chunk of
 // sweeps is launched back to back and the host reads the slots once per chunk.
 #include <algorithm>
 #include <climits>
@@ -58,13 +57,14 @@ __device__ __forceinline__ unsigned lanemask_lt()
 
 // flags[0]: malformed input, flags[1]: a row repeats a neighbour,
 // flags[2]: edge weights are not all bit-identical, flags[3]: max row length,
-// flags[4..5]: the largest positive weight (bits of the double), flags[8..11]:
+// flags[4..5]: the largest positive weight (bits of the double), flags[6]: an
+// edge id stands in two oriented slots (k_slot_counts), flags[8..11]:
 // the smallest and largest vertex weight (k_nw_bounds).
 // One warp per row (a hub's row is spread over the lanes).  A row outside
 // [0, S) or with end < begin is flagged and not read, so a malformed
 // adj_offset never leads to a read outside adj_target.
 __global__ void k_validate_rows(int N, int E, long long S, const int *off, const int *tgt, const int *eidx,
-                                int *deg, int *flags)
+                                int *__restrict__ deg, int *flags)
 {
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -97,7 +97,16 @@ __global__ void k_validate_rows(int N, int E, long long S, const int *off, const
         if (rmax) atomicMax(&flags[3], rmax);
     }
 }
-__global__ void k_validate_edges(int N, int E, const int *U, const int *V, const double *w, int *flags)
+// An edge's inputs in one 32-byte sector: the renumbering gathers them in random
+// order, a sector an array otherwise (28 M edges: 2.4 ms, 1.2 so).
+struct __align__(32) EdgeRec {
+    int u, v;
+    double w, d, unused;
+};
+
+__global__ void k_validate_edges(int N, int E, const int *__restrict__ U, const int *__restrict__ V,
+                                 const double *__restrict__ w, const double *__restrict__ d, int *flags,
+                                 EdgeRec *__restrict__ rec)
 {
     unsigned long long w0 = E > 0 ? (unsigned long long)__double_as_longlong(w[0]) : 0ULL;
     double wm = 0.0;
@@ -105,6 +114,7 @@ __global__ void k_validate_edges(int N, int E, const int *U, const int *V, const
         int u = U[e], v = V[e];
         if (u < 0 || u >= N || v < 0 || v >= N) atomicOr(&flags[0], 8);
         const double we = w[e];
+        rec[e] = EdgeRec{u, v, we, d[e], 0.0};
         if ((unsigned long long)__double_as_longlong(we) != w0) flags[2] = 1;
         wm = we > wm ? we : wm;
     }
@@ -202,116 +212,302 @@ __global__ void k_orient_count(int N, const int *off, const int *tgt, const int 
         if (lane == 0) ocnt[u] = c;
     }
 }
-__global__ void k_orient_fill(int N, const int *off, const int *tgt, const int *eidx, const int *deg,
-                              const long long *ooff, int *otgt, int *oeid, int *osrc)
+// A long row takes ROW_STRIPS strips at a time: one by one they are a chain of two
+// dependent loads each (a hub of 5,671 slots: 90 us, 30 so).
+constexpr int ROW_STRIPS = 8;
+template <int R>
+__device__ __forceinline__ void orient_strips(int u, unsigned long long ku, int b, int k0, int n, long long &o,
+                                              const int *__restrict__ tgt, const int *__restrict__ eidx,
+                                              const int *__restrict__ deg, int *__restrict__ otgt,
+                                              int *__restrict__ oeid, int *__restrict__ osrc)
 {
     const int lane = threadIdx.x & 31;
+    int x[R], id[R];
+    bool keep[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int k = k0 + 32 * r + lane;
+        x[r] = k < n ? tgt[b + k] : u;              // (no vertex ranks above itself)
+        id[r] = k < n ? eidx[b + k] : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) keep[r] = rank_key(deg, x[r]) > ku;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const unsigned m = __ballot_sync(0xffffffffu, keep[r]);
+        if (keep[r]) {
+            const long long at = o + __popc(m & lanemask_lt());
+            otgt[at] = x[r];
+            oeid[at] = id[r];
+            osrc[at] = u;
+        }
+        o += __popc(m);
+    }
+}
+
+__global__ void k_orient_fill(int N, const int *__restrict__ off, const int *__restrict__ tgt,
+                              const int *__restrict__ eidx, const int *__restrict__ deg,
+                              const long long *__restrict__ ooff, int *__restrict__ otgt, int *__restrict__ oeid,
+                              int *__restrict__ osrc)
+{
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < N; u += nw) {
         const unsigned long long ku = rank_key(deg, u);
         long long o = ooff[u];
-        const int b = off[u], e = off[u + 1];
-        for (int q0 = b; q0 < e; q0 += 32) {
-            const int q = q0 + lane;
-            int x = 0;
-            bool keep = false;
-            if (q < e) {
-                x = tgt[q];
-                keep = rank_key(deg, x) > ku;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) {
-                const long long at = o + __popc(m & lanemask_lt());
-                otgt[at] = x;
-                oeid[at] = eidx[q];
-                osrc[at] = u;
-            }
-            o += __popc(m);
-        }
+        const int b = off[u], n = off[u + 1] - b;
+        int k = 0;
+        for (; n - k > 128; k += 32 * ROW_STRIPS)
+            orient_strips<ROW_STRIPS>(u, ku, b, k, n, o, tgt, eidx, deg, otgt, oeid, osrc);
+        for (; k < n; k += 32) orient_strips<1>(u, ku, b, k, n, o, tgt, eidx, deg, otgt, oeid, osrc);
     }
 }
 
-// Each oriented edge a->b intersects out(a) with out(b) (both ascending by id).
-// A common c closes the triangle {a,b,c}; each of its three edges receives
-// the pair of the other two (the order inside a pair is irrelevant: the term
-// is their sum).
-// The pairs an oriented edge finds for itself go to the head of its own list
-// (own[eab] of them, counted in the first pass), without atomics; the pairs
-// it finds for its triangles' other two edges go through their cursors,
-// which start after those heads.  Two rows of very different lengths are
-// intersected by binary searches of the short row's ids in the long one
-// (a merge walk would step through the whole long row).
+// Triangles {a, b, c}: for each oriented edge a->b the members of out(b) that
+// are in out(a) (rows ascend by id).  Each of a triangle's edges receives the
+// pair of the other two; the order inside a pair and of the pairs is irrelevant
+// (the term is their sum, and the sums are exact).  This pass counts per oriented
+// slot and lists the triangles' slots; their pairs are written in the new
+// numbering, where an owner's lists lie next to each other, from the list
+// (k_triangle_pairs) or, where a dense graph overflows it, by a second pass.
+// A warp takes 32 oriented edges.  For each owner among them it lays out(a)
+// down as a 1024-bit filter, a word a lane, and a hash table of positions (a row
+// of more than TRI_HASH / 2 is searched instead), reads the rows out(b) in
+// coalesced strips and looks up only what passes the filter.  A thread per edge
+// that walks two rows touches a cache line a lane on every step.  Bound by
+// instruction issue (87 %).  28 M power-law edges: this pass 5.9 ms and the list's
+// pairs 1.4, where two passes of a thread per edge took 5.2 and 9.3 and the
+// pairs' renumbering 1.2; 200,003 edges: 59 us for 118.
+constexpr int TRI_HASH = 1024;
+constexpr int TRI_CHUNK = 128;        // list entries a warp reserves at a time
+struct TriList {
+    int *ab, *ac, *bc;                // oriented slots; ab < 0: no triangle
+    long long cap;
+    unsigned long long *total;        // entries reserved
+};
+__device__ __forceinline__ unsigned filter_bit(int x) { return ((unsigned)x * 2654435769u) >> 22; }
+
 template <bool FILL>
-__global__ void k_triangles(long long M, const long long *ooff, const int *otgt, const int *oeid,
-                            const int *osrc, int *cnt, int *own_cnt, const long long *ioff,
-                            unsigned long long *cursor, int2 *pairs)
+__global__ void __launch_bounds__(256) k_triangles(int M, const long long *ooff, const int *otgt, const int *oeid,
+                                                   const int *osrc, int *cntq, TriList list,
+                                                   unsigned long long *cursor, int2 *pairs)
+{
+    __shared__ unsigned sw[8][32];
+    __shared__ __align__(16) unsigned short sh[8][TRI_HASH];
+    const int lane = threadIdx.x & 31;
+    unsigned *fw = sw[threadIdx.x >> 5];
+    unsigned short *table = sh[threadIdx.x >> 5];
+    long long pos = 0;                              // this warp's place in the list
+    int left = 0;
+    const int units = (M + 31) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    for (int unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < units; unit += warps) {
+        const int q = unit * 32 + lane;
+        int a = -1, pa = 0, la = 0, pb = 0, lb = 0;
+        if (q < M) {
+            a = osrc[q];
+            const int b = otgt[q];
+            pa = (int)ooff[a];
+            la = (int)ooff[a + 1] - pa;
+            pb = (int)ooff[b];
+            lb = (int)ooff[b + 1] - pb;
+        }
+        // an owner of one oriented edge closes no triangle
+        unsigned rem = __ballot_sync(0xffffffffu, la > 1 && lb > 0);
+        int own = 0;                                // this lane's edge: its triangles (as a->b)
+        while (rem) {
+            const int lead = __ffs(rem) - 1;
+            const int A = __shfl_sync(0xffffffffu, a, lead);
+            const int rb = __shfl_sync(0xffffffffu, pa, lead), rn = __shfl_sync(0xffffffffu, la, lead);
+            unsigned seg = rem & __ballot_sync(0xffffffffu, a == A);
+            rem &= ~seg;
+            const bool hashed = rn <= TRI_HASH / 2;
+            fw[lane] = 0u;
+            if (hashed)
+                for (int k = lane; k < TRI_HASH / 8; k += 32) reinterpret_cast<uint4 *>(table)[k] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            for (int k = lane; k < rn; k += 32) {
+                unsigned h = filter_bit(otgt[rb + k]);
+                atomicOr(&fw[h >> 5], 1u << (h & 31));
+                if (hashed)
+                    while (atomicCAS(&table[h], (unsigned short)0, (unsigned short)(k + 1)) != 0) h = (h + 1) & (TRI_HASH - 1);
+            }
+            __syncwarp();
+            const unsigned f = fw[lane];
+            __syncwarp();
+            // the strips of the owner's rows out(b), one read ahead
+            int i = __ffs(seg) - 1;
+            int rp = __shfl_sync(0xffffffffu, pb, i), rl = __shfl_sync(0xffffffffu, lb, i), o = 0;
+            int x = lane < rl ? otgt[rp + lane] : -1;
+            while (seg) {
+                const int ci = i, cp = rp + o, cx = x;
+                o += 32;
+                if (o >= rl) {
+                    seg &= seg - 1;
+                    o = 0;
+                    if (seg) {
+                        i = __ffs(seg) - 1;
+                        rp = __shfl_sync(0xffffffffu, pb, i);
+                        rl = __shfl_sync(0xffffffffu, lb, i);
+                    }
+                }
+                if (seg) x = o + lane < rl ? otgt[rp + o + lane] : -1;
+                const unsigned h = filter_bit(cx);
+                bool hit = (__shfl_sync(0xffffffffu, f, (int)(h >> 5)) >> (h & 31)) & 1u;
+                hit = hit && cx >= 0;
+                if (!__any_sync(0xffffffffu, hit)) continue;
+                int at = rb;                        // cx's place in out(a)
+                if (hit && hashed) {
+                    unsigned slot = h;
+                    int k;
+                    while ((k = table[slot]) != 0 && otgt[rb + k - 1] != cx) slot = (slot + 1) & (TRI_HASH - 1);
+                    at += k - 1;
+                    hit = k != 0;
+                } else if (hit) {
+                    int n = rn;
+                    while (n > 0) {
+                        const int half = n >> 1;
+                        if (otgt[at + half] < cx) {
+                            at += half + 1;
+                            n -= half + 1;
+                        } else {
+                            n = half;
+                        }
+                    }
+                    hit = at < rb + rn && otgt[at] == cx;
+                }
+                const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                if (!hits) continue;
+                if (!FILL) {
+                    const int nh = __popc(hits);
+                    if (lane == ci) own += nh;
+                    if (left < nh) {
+                        if (lane < left && pos + lane < list.cap) list.ab[pos + lane] = -1;
+                        if (lane == 0) pos = (long long)atomicAdd(list.total, (unsigned long long)TRI_CHUNK);
+                        pos = __shfl_sync(0xffffffffu, pos, 0);
+                        left = TRI_CHUNK;
+                    }
+                    if (hit) {
+                        atomicAdd(&cntq[at], 1);
+                        atomicAdd(&cntq[cp + lane], 1);
+                        const long long t = pos + __popc(hits & lanemask_lt());
+                        if (t < list.cap) {
+                            list.ab[t] = unit * 32 + ci;
+                            list.ac[t] = at;
+                            list.bc[t] = cp + lane;
+                        }
+                    }
+                    pos += nh;
+                    left -= nh;
+                } else {
+                    const int eab = oeid[unit * 32 + ci];
+                    unsigned long long base = 0;
+                    if (lane == 0) base = atomicAdd(&cursor[eab], (unsigned long long)__popc(hits));
+                    if (hit) {
+                        const int eac = oeid[at], ebc = oeid[cp + lane];
+                        const unsigned long long oc = atomicAdd(&cursor[eac], 1ULL), ob = atomicAdd(&cursor[ebc], 1ULL);
+                        pairs[oc] = make_int2(eab, ebc);
+                        pairs[ob] = make_int2(eab, eac);
+                    }
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (hit) pairs[base + __popc(hits & lanemask_lt())] = make_int2(oeid[at], oeid[cp + lane]);
+                }
+            }
+        }
+        if (!FILL && own) atomicAdd(&cntq[q], own);
+    }
+    if (!FILL)
+        for (int k = lane; k < left; k += 32)
+            if (pos + k < list.cap) list.ab[pos + k] = -1;
+}
+
+// the listed triangles' pairs (oeid: new ids)
+__global__ void k_triangle_pairs(TriList list, const int *__restrict__ oeid, unsigned long long *cursor,
+                                 int2 *__restrict__ pairs)
+{
+    const long long n = (long long)*list.total;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int ab = list.ab[t];
+        if (ab < 0) continue;
+        const int eab = oeid[ab], eac = oeid[list.ac[t]], ebc = oeid[list.bc[t]];
+        const unsigned long long ob = atomicAdd(&cursor[eab], 1ULL), oc = atomicAdd(&cursor[eac], 1ULL),
+                                 ox = atomicAdd(&cursor[ebc], 1ULL);
+        pairs[ob] = make_int2(eac, ebc);
+        pairs[oc] = make_int2(eab, ebc);
+        pairs[ox] = make_int2(eab, eac);
+    }
+}
+
+// pairs of each edge, from the counts of its oriented slots; *twice is set when
+// an edge id stands in more than one
+__global__ void k_slot_counts(int M, const int *oeid, const int *cntq, int *cnt, unsigned *seen, int *twice)
 {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < M;
          q += (long long)gridDim.x * blockDim.x) {
-        int a = osrc[q], b = otgt[q], eab = oeid[q];
-        long long pa = ooff[a], pa_end = ooff[a + 1];
-        long long pb = ooff[b], pb_end = ooff[b + 1];
-        int own = 0;                           // this edge's triangles so far
-        const long long head = FILL ? ioff[eab] : 0;
-        auto found = [&](int eac, int ebc) {
-            if (!FILL) {
-                ++own;
-                atomicAdd(&cnt[eac], 1);
-                atomicAdd(&cnt[ebc], 1);
-            } else {
-                pairs[head + own++] = make_int2(eac, ebc);
-                pairs[atomicAdd(&cursor[eac], 1ULL)] = make_int2(eab, ebc);
-                pairs[atomicAdd(&cursor[ebc], 1ULL)] = make_int2(eab, eac);
-            }
-        };
-        const long long la = pa_end - pa, lb = pb_end - pb;
-        const long long ls = la < lb ? la : lb, ll = la < lb ? lb : la;
-        if (ls > 0 && ls * (64 - __clzll(ll)) < ll) {
-            const bool a_short = la <= lb;
-            const long long s0 = a_short ? pa : pb, s1 = a_short ? pa_end : pb_end;
-            long long lo = a_short ? pb : pa;
-            const long long l1 = a_short ? pb_end : pa_end;
-            for (long long i = s0; i < s1 && lo < l1; ++i) {
-                const int x = otgt[i];
-                long long L = lo, R = l1;              // first id >= x in the long row
-                while (L < R) {
-                    const long long mid = (L + R) >> 1;
-                    if (otgt[mid] < x) L = mid + 1;
-                    else R = mid;
-                }
-                lo = L;
-                if (L < l1 && otgt[L] == x) {
-                    found(oeid[a_short ? i : L], oeid[a_short ? L : i]);
-                    ++lo;
-                }
-            }
-        } else {
-            while (pa < pa_end && pb < pb_end) {
-                int x = otgt[pa], y = otgt[pb];
-                if (x == y) {
-                    found(oeid[pa], oeid[pb]);
-                    ++pa;
-                    ++pb;
-                } else if (x < y) {
-                    ++pa;
-                } else {
-                    ++pb;
-                }
-            }
-        }
-        if (!FILL) {
-            own_cnt[eab] = own;                // each edge is one oriented edge
-            if (own) atomicAdd(&cnt[eab], own);
+        const int e = oeid[q];
+        if (atomicOr(&seen[e >> 5], 1u << (e & 31)) >> (e & 31) & 1u) *twice = 1;
+        if (cntq[q]) atomicAdd(&cnt[e], cntq[q]);
+    }
+}
+
+__global__ void k_renumber(int M, const int *einv, int *oeid)
+{
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < M;
+         q += (long long)gridDim.x * blockDim.x)
+        oeid[q] = einv[oeid[q]];
+}
+
+// Edges of a large graph by owner (the endpoint of lower rank) when every edge
+// is one oriented slot: the oriented rows are the owners' edge lists already,
+// so the new ids follow from two scans over the owners in the new vertex order,
+// the edges without common neighbours first.  (See k_edge_keys, which sorts, for
+// why.)  A warp per owner; on 28 M edges 1.9 ms where keys and sort took 6.
+__global__ void k_owner_counts(int N, const int *vperm, const long long *ooff, const int *cntq, int *none, int *some)
+{
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += nw) {
+        const int u = vperm[i];
+        const int b = (int)ooff[u], e = (int)ooff[u + 1];
+        int c = 0;
+        for (int q = b + lane; q < e; q += 32) c += cntq[q] > 0;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) {
+            some[i] = c;
+            none[i] = e - b - c;
         }
     }
 }
 
-// each edge's cursor: the start of its pair list past its own pairs
-__global__ void k_cursor_init(long long n, const long long *ioff, const int *own_cnt, unsigned long long *cursor)
+// new ids of the owners' edges: eperm, einv and the pair counts in the new
+// order; oeid itself is renumbered
+__global__ void k_owner_place(int N, int e0, const int *__restrict__ vperm, const long long *__restrict__ ooff,
+                              const int *__restrict__ cntq, const long long *__restrict__ none,
+                              const long long *__restrict__ some, int *oeid, int *__restrict__ eperm,
+                              int *__restrict__ einv, int *__restrict__ ncnt)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        cursor[i] = (unsigned long long)(ioff[i] + own_cnt[i]);
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += nw) {
+        const int u = vperm[i];
+        const int b = (int)ooff[u], e = (int)ooff[u + 1];
+        int at0 = (int)none[i], at1 = e0 + (int)some[i];
+        for (int q0 = b; q0 < e; q0 += 32) {
+            const int q = q0 + lane;
+            const int c = q < e ? cntq[q] : 0;
+            const unsigned live = __ballot_sync(0xffffffffu, q < e), m = __ballot_sync(0xffffffffu, c > 0);
+            if (q < e) {
+                const unsigned below = lanemask_lt();
+                const int j = c > 0 ? at1 + __popc(m & below) : at0 + __popc(live & ~m & below);
+                const int id = oeid[q];
+                eperm[j] = id;
+                einv[id] = j;
+                ncnt[j] = c;
+                oeid[q] = j;
+            }
+            at1 += __popc(m);
+            at0 += __popc(live & ~m);
+        }
+    }
 }
 
 // ---- binning (terms per item) and renumbering ----
@@ -586,7 +782,7 @@ __global__ void __launch_bounds__(SORT_BLK_THR) k_sort_rows_blk(int lo, int hi, 
     }
 }
 
-__global__ void k_gather_seg(int n, const int *perm, const int *len, int *out)
+__global__ void k_gather_len(int n, const int *perm, const int *len, int *out)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = len[perm[i]];
 }
@@ -596,15 +792,10 @@ __global__ void k_fix_inv(int n, int base, const int *perm, int *inv)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) inv[perm[base + i]] = base + i;
 }
 
-__global__ void k_gather_deg(int N, const int *vperm, const int *deg, int *ndeg)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-        ndeg[i] = deg[vperm[i]];
-}
-
 // one warp per (renumbered) vertex: copy its row with renumbered edge ids
-__global__ void k_new_rows(int N, const int *vperm, const int *off, const int *eidx, const int *einv,
-                           const long long *row_off, int *row_eid, const double *nw_in, double *nw_out)
+__global__ void k_new_rows(int N, const int *__restrict__ vperm, const int *__restrict__ off,
+                           const int *__restrict__ eidx, const int *__restrict__ einv,
+                           const long long *__restrict__ row_off, int *__restrict__ row_eid)
 {
     int lane = threadIdx.x & 31;
     int warps = (gridDim.x * blockDim.x) >> 5;
@@ -612,23 +803,35 @@ __global__ void k_new_rows(int N, const int *vperm, const int *off, const int *e
         int u = vperm[i];
         int b = off[u], n = off[u + 1] - b;
         long long o = row_off[i];
-        for (int k = lane; k < n; k += 32) row_eid[o + k] = einv[eidx[b + k]];
-        if (lane == 0) nw_out[i] = nw_in[u];
+        int k = lane;
+        for (; k + 32 * (ROW_STRIPS - 1) < n; k += 32 * ROW_STRIPS) {
+            int id[ROW_STRIPS];
+#pragma unroll
+            for (int r = 0; r < ROW_STRIPS; ++r) id[r] = eidx[b + k + 32 * r];
+#pragma unroll
+            for (int r = 0; r < ROW_STRIPS; ++r) id[r] = einv[id[r]];
+#pragma unroll
+            for (int r = 0; r < ROW_STRIPS; ++r) row_eid[o + k + 32 * r] = id[r];
+        }
+        for (; k < n; k += 32) row_eid[o + k] = einv[eidx[b + k]];
     }
 }
 
-__global__ void k_new_edges(int E, const int *eperm, const int *U, const int *V, const int *vinv,
-                            const double *w, const double *d, const int *cnt, int *eu, int *ev,
-                            double *wn, double *d0, double *p0, int *ncnt)
+__global__ void k_new_nw(int N, const int *vperm, const double *nw_in, double *nw_out)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) nw_out[i] = nw_in[vperm[i]];
+}
+
+__global__ void k_new_edges(int E, const int *__restrict__ eperm, const EdgeRec *__restrict__ rec,
+                            const int *__restrict__ vinv, int *__restrict__ eu, int *__restrict__ ev,
+                            double *__restrict__ wn, double *__restrict__ d0, double *__restrict__ p0)
 {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < E; j += gridDim.x * blockDim.x) {
-        int e = eperm[j];
-        eu[j] = vinv[U[e]];
-        ev[j] = vinv[V[e]];
-        double we = w[e], de = d[e];
-        d0[j] = de;
-        if (wn) { wn[j] = we; p0[j] = dmul(we, de); }
-        ncnt[j] = cnt[e];
+        const EdgeRec r = rec[eperm[j]];
+        eu[j] = vinv[r.u];
+        ev[j] = vinv[r.v];
+        d0[j] = r.d;
+        if (wn) { wn[j] = r.w; p0[j] = dmul(r.w, r.d); }
     }
 }
 
@@ -804,11 +1007,15 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     // pairs unless the triangle listing (CSR only) makes them.
     bool uniform = true;
     double w_max = 0.0, nw_lo = 1.0, nw_hi = 1.0;      // NULL vertex weights mean all 1.0
+    bool edges_valid = false;
+    DevBuf<EdgeRec> d_rec;
     auto validate_edges = [&]() -> Status {
         DRESS_TRY(edge_up.join());
+        DRESS_TRY(d_rec.alloc((size_t)E, st));
         const auto v0 = std::chrono::steady_clock::now();
         count_launch(), k_validate_edges<<<grid_for(E, 256, 16 * sms), 256, 0, st>>>(N, E, d_U.get(), d_V.get(),
-                                                                                      d_w.get(), d_flags.get());
+                                                                                      d_w.get(), d_d.get(),
+                                                                                      d_flags.get(), d_rec.get());
         if (g->NW && N)
             count_launch(), k_nw_bounds<<<grid_for(N, 256, 16 * sms), 256, 0, st>>>(
                 N, d_nw.get(), (unsigned long long *)(d_flags.get() + 8));
@@ -817,6 +1024,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
         t_valid += ms_since(v0);
         if (flags[0]) return Status::Err(DRESSX_EINVAL, "malformed graph (CSR or edge endpoints out of range)");
+        edges_valid = true;
         uniform = flags[2] == 0;
         std::memcpy(&w_max, flags + 4, sizeof w_max);
         if (g->NW && N) {
@@ -832,23 +1040,18 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     // ---- common-neighbour tables (original edge ids) -------------------------
     DevBuf<long long> d_ioff_old, d_scan_tmp;
     DevBuf<int2> d_pairs_old;
-    // the oriented rows of the triangle listing, alive until its fill is joined
-    DevBuf<int> d_ocnt, d_otgt, d_oeid, d_osrc, d_own;
+    // the oriented rows of the triangle listing, alive until its second pass
+    DevBuf<int> d_ocnt, d_otgt, d_oeid, d_osrc, d_cntq;
     DevBuf<long long> d_ooff;
-    DevBuf<unsigned long long> d_cursor;
-    // Declared after the buffers the side-stream fill reads, so that on an
-    // early return it waits for the fill before they are freed.
-    struct SideFill {
-        cudaStream_t side;
-        bool pending = false;
-        ~SideFill()
-        {
-            if (pending) cudaStreamSynchronize(side);
-        }
-    } fill{ctx.side};
-    DRESS_TRY(d_ioff_old.alloc((size_t)E + 1, st));
+    DevBuf<int> d_tri;
+    DevBuf<unsigned long long> d_tri_total;
+    TriList tri{};
+    unsigned long long listed = 0;
+    int tri_blocks = 1;
+    if (!tri_path) DRESS_TRY(d_ioff_old.alloc((size_t)E + 1, st));
     DRESS_TRY(d_scan_tmp.alloc(scan_tmp_elems((long long)(S > E ? S : E) + N + 1), st));
-    long long T = 0;
+    long long T = 0, M = 0;
+    int tg = 1;                              // blocks over the oriented edges
     const int eg = (int)grid_for(E, 256, 32 * sms);
     if (g->precompute_intercepts && g->intercept_offset) {
         DevBuf<int> d_io, d_ux, d_vx;
@@ -868,41 +1071,42 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         DRESS_TRY(d_pairs_old.alloc((size_t)(T > 0 ? T : 1), st));
         count_launch(), k_given_pairs<<<eg, 256, 0, st>>>(E, d_io.get(), d_ux.get(), d_vx.get(), d_ioff_old.get(),
                                           d_pairs_old.get(), d_flags.get());
-    } else if (g->variant == DRESS_VARIANT_UNDIRECTED && !dup) {
+    } else if (tri_path) {
         DRESS_TRY(d_ocnt.alloc((size_t)N, st));
         DRESS_TRY(d_ooff.alloc((size_t)N + 1, st));
-        DRESS_TRY(d_otgt.alloc((size_t)(S > 0 ? S : 1), st));
-        DRESS_TRY(d_oeid.alloc((size_t)(S > 0 ? S : 1), st));
-        DRESS_TRY(d_osrc.alloc((size_t)(S > 0 ? S : 1), st));
         const int vg = (int)grid_for((long long)N * 32, 256, 32 * sms);     // a warp per row
         count_launch(), k_orient_count<<<vg, 256, 0, st>>>(N, d_off.get(), d_tgt.get(), d_deg.get(), d_ocnt.get());
         DRESS_TRY(exclusive_scan_i32(d_ocnt.get(), d_ooff.get(), N, d_scan_tmp.get(), st));
+        DRESS_CUDA_TRY(counted_memcpy(&M, d_ooff.get() + N, sizeof(M), cudaMemcpyDeviceToHost, st));
+        DRESS_CUDA_TRY(cudaMemsetAsync(d_cnt.get(), 0, (size_t)E * sizeof(int), st));   // self loops are never oriented
+        DRESS_CUDA_TRY(cudaStreamSynchronize(st));
+        const size_t slots = (size_t)(M > 0 ? M : 1);
+        DRESS_TRY(d_otgt.alloc(slots, st));
+        DRESS_TRY(d_oeid.alloc(slots, st));
+        DRESS_TRY(d_osrc.alloc(slots, st));
         count_launch(), k_orient_fill<<<vg, 256, 0, st>>>(N, d_off.get(), d_tgt.get(), d_eidx.get(), d_deg.get(),
                                           d_ooff.get(), d_otgt.get(), d_oeid.get(), d_osrc.get());
-        long long M = 0;
-        DRESS_CUDA_TRY(counted_memcpy(&M, d_ooff.get() + N, sizeof(M), cudaMemcpyDeviceToHost, st));
-        DRESS_CUDA_TRY(cudaMemsetAsync(d_cnt.get(), 0, (size_t)E * sizeof(int), st));
-        DRESS_CUDA_TRY(cudaStreamSynchronize(st));
-        const int tg = (int)grid_for(M, 256, 64 * sms);
-        DRESS_TRY(d_own.alloc((size_t)(E > 0 ? E : 1), st));
-        DRESS_CUDA_TRY(cudaMemsetAsync(d_own.get(), 0, (size_t)E * sizeof(int), st));   // self loops are never oriented
-        count_launch(), k_triangles<false><<<tg, 256, 0, st>>>(M, d_ooff.get(), d_otgt.get(), d_oeid.get(), d_osrc.get(),
-                                               d_cnt.get(), d_own.get(), nullptr, nullptr, nullptr);
-        DRESS_TRY(exclusive_scan_i32(d_cnt.get(), d_ioff_old.get(), E, d_scan_tmp.get(), st));
-        DRESS_CUDA_TRY(counted_memcpy(&T, d_ioff_old.get() + E, sizeof(T), cudaMemcpyDeviceToHost, st));
-        DRESS_CUDA_TRY(cudaStreamSynchronize(st));
-        DRESS_TRY(d_pairs_old.alloc((size_t)(T > 0 ? T : 1), st));
-        DRESS_TRY(d_cursor.alloc((size_t)E, st));
-        count_launch(), k_cursor_init<<<eg, 256, 0, st>>>(E, d_ioff_old.get(), d_own.get(), d_cursor.get());
-        // The fill runs on the side stream, beside the edge validation, the
-        // bins and the edge renumbering, which need only the counts; the main
-        // stream joins it before the first read of the pairs (k_new_pairs).
-        DRESS_CUDA_TRY(cudaEventRecord(ctx.fork, st));
-        DRESS_CUDA_TRY(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
-        fill.pending = true;
-        count_launch(), k_triangles<true><<<tg, 256, 0, ctx.side>>>(M, d_ooff.get(), d_otgt.get(), d_oeid.get(),
-                                                                    d_osrc.get(), nullptr, nullptr, d_ioff_old.get(),
-                                                                    d_cursor.get(), d_pairs_old.get());
+        DRESS_TRY(d_cntq.alloc((size_t)(M > 0 ? M : 1), st));
+        DRESS_CUDA_TRY(cudaMemsetAsync(d_cntq.get(), 0, (size_t)M * sizeof(int), st));
+        tg = (int)grid_for(M, 256, 32 * sms);
+        // room for two triangles a slot (a power-law graph of 28 M edges closes
+        // 1.2) and what the warps leave open
+        tri_blocks = (int)grid_for(M, 256, 6 * sms);
+        tri.cap = 2 * M + (long long)tri_blocks * 8 * TRI_CHUNK;
+        DRESS_TRY(d_tri.alloc(3 * (size_t)tri.cap, st));
+        DRESS_TRY(d_tri_total.alloc(1, st));
+        DRESS_CUDA_TRY(cudaMemsetAsync(d_tri_total.get(), 0, sizeof(unsigned long long), st));
+        tri.ab = d_tri.get();
+        tri.ac = tri.ab + tri.cap;
+        tri.bc = tri.ac + tri.cap;
+        tri.total = d_tri_total.get();
+        count_launch(), k_triangles<false><<<tri_blocks, 256, 0, st>>>((int)M, d_ooff.get(), d_otgt.get(), nullptr,
+                                                                       d_osrc.get(), d_cntq.get(), tri, nullptr, nullptr);
+        DevBuf<unsigned> d_seen;
+        DRESS_TRY(d_seen.alloc((size_t)E / 32 + 1, st));
+        DRESS_CUDA_TRY(cudaMemsetAsync(d_seen.get(), 0, ((size_t)E / 32 + 1) * sizeof(unsigned), st));
+        count_launch(), k_slot_counts<<<tg, 256, 0, st>>>((int)M, d_oeid.get(), d_cntq.get(), d_cnt.get(),
+                                                          d_seen.get(), d_flags.get() + 6);
     } else {
         count_launch(), k_merge_intercepts<false><<<eg, 256, 0, st>>>(E, d_U.get(), d_V.get(), d_off.get(), d_tgt.get(),
                                                        d_eidx.get(), d_cnt.get(), nullptr, nullptr);
@@ -915,7 +1119,6 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
                                                       d_pairs_old.get());
     }
     DRESS_CUDA_TRY(cudaGetLastError());
-    if (tri_path) DRESS_TRY(validate_edges());
     d_tgt.release();
 
     // ---- bins and renumbering ---------------------------------------------------
@@ -940,7 +1143,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DRESS_CUDA_TRY(counted_memcpy(bc.data(), d_bc.get(), 2 * NF * sizeof(int), cudaMemcpyDeviceToHost, st));
     DRESS_CUDA_TRY(counted_memcpy(flags, d_flags.get(), sizeof(flags), cudaMemcpyDeviceToHost, st));
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));
-    const double t_pairs = ms_since(t0);
+    const double t_pairs = ms_since(t0), early_ms = edge_up.wait_ms + t_valid;   // (part of it)
     if (flags[0]) return Status::Err(DRESSX_EINVAL, "malformed intercept tables");
     // fine ranges (cursors), then the coarse bins they make up
     std::vector<int> cur(2 * NF);
@@ -968,14 +1171,17 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     }
     DRESS_CUDA_TRY(counted_memcpy(d_bc.get() + 2 * NF, cur.data(), 2 * NF * sizeof(int), cudaMemcpyHostToDevice, st));
     count_launch(), k_bin_scatter<<<vg, 256, 0, st>>>(N, d_deg.get(), d_bc.get() + 2 * NF, d_vperm.get(), d_vinv.get());
-    // Edges of a large graph: one stable radix sort on (any pairs, owner,
-    // other endpoint), for the locality of the sweeps' gathers.  A small
+    // Edges of a large graph in the order (any pairs, owner), for the locality
+    // of the sweeps' gathers: from the oriented rows when every edge is one of
+    // their slots, else one stable radix sort.  A small
     // graph's sweeps are bound by launch latency and its arrays sit in L2, so
     // it keeps the one-pass scatter (the sort's passes cost more than they save).
     const bool locality = E >= LOCALITY_MIN_EDGES;
     if (!locality)
         count_launch(), k_bin_scatter<<<eg, 256, 0, st>>>(E, d_cnt.get(), d_bc.get() + 3 * NF, d_eperm.get(), d_einv.get());
-    if (locality) {
+    const bool by_owner = locality && tri_path && M == E && !flags[6];
+    if (locality && !by_owner) {
+        if (tri_path) DRESS_TRY(validate_edges());   // the keys read the edge arrays
         DevBuf<unsigned long long> k0, k1;
         DevBuf<unsigned> v0, v1;
         DRESS_TRY(k0.alloc((size_t)E, st));
@@ -1004,7 +1210,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
             if (n < 2) continue;
             DevBuf<int> d_len;
             DRESS_TRY(d_len.alloc((size_t)n, st));
-            count_launch(), k_gather_seg<<<grid_for(n, 256, 64 * sms), 256, 0, st>>>(n, g2.perm + g2.b0, g2.len, d_len.get());
+            count_launch(), k_gather_len<<<grid_for(n, 256, 64 * sms), 256, 0, st>>>(n, g2.perm + g2.b0, g2.len, d_len.get());
             std::vector<int> perm((size_t)n), len((size_t)n), idx((size_t)n);
             DRESS_CUDA_TRY(counted_memcpy(perm.data(), g2.perm + g2.b0, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st));
             DRESS_CUDA_TRY(counted_memcpy(len.data(), d_len.get(), (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1023,15 +1229,30 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DevBuf<long long> d_row_off, d_ioff;
     DevBuf<double> d_nwi, d_wi, d_dbuf, d_pbuf, d_vd;
     DevBuf<int2> d_pairs;
+    DRESS_TRY(d_ncnt.alloc((size_t)E, st));
+    if (by_owner) {
+        DevBuf<int> d_none, d_some;
+        DevBuf<long long> d_none_off, d_some_off;
+        DRESS_TRY(d_none.alloc((size_t)N, st));
+        DRESS_TRY(d_some.alloc((size_t)N, st));
+        DRESS_TRY(d_none_off.alloc((size_t)N + 1, st));
+        DRESS_TRY(d_some_off.alloc((size_t)N + 1, st));
+        const int wg = (int)grid_for((long long)N * 32, 256, 64 * sms);
+        count_launch(), k_owner_counts<<<wg, 256, 0, st>>>(N, d_vperm.get(), d_ooff.get(), d_cntq.get(), d_none.get(),
+                                                           d_some.get());
+        DRESS_TRY(exclusive_scan_i32(d_none.get(), d_none_off.get(), N, d_scan_tmp.get(), st));
+        DRESS_TRY(exclusive_scan_i32(d_some.get(), d_some_off.get(), N, d_scan_tmp.get(), st));
+        count_launch(), k_owner_place<<<wg, 256, 0, st>>>(N, eb.count(B0), d_vperm.get(), d_ooff.get(), d_cntq.get(),
+                                                          d_none_off.get(), d_some_off.get(), d_oeid.get(),
+                                                          d_eperm.get(), d_einv.get(), d_ncnt.get());
+    }
     DRESS_TRY(d_ndeg.alloc((size_t)N, st));
     DRESS_TRY(d_row_off.alloc((size_t)N + 1, st));
     DRESS_TRY(d_row_eid.alloc((size_t)(S > 0 ? S : 1), st));
-    DRESS_TRY(d_nwi.alloc((size_t)N, st));
-    count_launch(), k_gather_deg<<<vg, 256, 0, st>>>(N, d_vperm.get(), d_deg.get(), d_ndeg.get());
+    count_launch(), k_gather_len<<<vg, 256, 0, st>>>(N, d_vperm.get(), d_deg.get(), d_ndeg.get());
     DRESS_TRY(exclusive_scan_i32(d_ndeg.get(), d_row_off.get(), N, d_scan_tmp.get(), st));
     count_launch(), k_new_rows<<<grid_for((long long)N * 32, 256, 64 * sms), 256, 0, st>>>(
-        N, d_vperm.get(), d_off.get(), d_eidx.get(), d_einv.get(), d_row_off.get(), d_row_eid.get(),
-        d_nw.get(), d_nwi.get());
+        N, d_vperm.get(), d_off.get(), d_eidx.get(), d_einv.get(), d_row_off.get(), d_row_eid.get());
     if (locality) {                          // rows in edge-id order (vertex bins: thread, warp, block)
         const int t0 = vb.start[B2], t1 = vb.start[BMED], w1 = vb.start[BBLOCK], b1 = vb.start[BBIG];
         if (t1 > t0)
@@ -1047,18 +1268,8 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     d_eidx.release();
     d_ndeg.release();
 
-    DRESS_TRY(d_eu.alloc((size_t)E, st));
-    DRESS_TRY(d_ev.alloc((size_t)E, st));
-    DRESS_TRY(d_ncnt.alloc((size_t)E, st));
-    DRESS_TRY(d_dbuf.alloc(2 * (size_t)E, st));
-    if (!uniform) {
-        DRESS_TRY(d_wi.alloc((size_t)E, st));
-        DRESS_TRY(d_pbuf.alloc(2 * (size_t)E, st));
-    }
-    count_launch(), k_new_edges<<<eg, 256, 0, st>>>(E, d_eperm.get(), d_U.get(), d_V.get(), d_vinv.get(), d_w.get(),
-                                    d_d.get(), d_cnt.get(), d_eu.get(), d_ev.get(),
-                                    uniform ? nullptr : d_wi.get(), d_dbuf.get(),
-                                    uniform ? nullptr : d_pbuf.get(), d_ncnt.get());
+    if (!by_owner)
+        count_launch(), k_gather_len<<<eg, 256, 0, st>>>(E, d_eperm.get(), d_cnt.get(), d_ncnt.get());
     DRESS_TRY(d_ioff.alloc((size_t)E + 1, st));
     DRESS_TRY(exclusive_scan_i32(d_ncnt.get(), d_ioff.get(), E, d_scan_tmp.get(), st));
     // The edges with common neighbours listed by size class (EdgeClasses):
@@ -1103,15 +1314,29 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         }
     }
     ec.list = d_elist.get();
-    DRESS_TRY(d_pairs.alloc((size_t)(T > 0 ? T : 1), st));
-    if (fill.pending) {                      // the pairs of the triangle listing are complete
-        DRESS_CUDA_TRY(cudaEventRecord(ctx.join, ctx.side));
-        DRESS_CUDA_TRY(cudaStreamWaitEvent(st, ctx.join, 0));
-        fill.pending = false;
-        d_otgt.release(); d_oeid.release(); d_osrc.release(); d_ooff.release(); d_ocnt.release();
-        d_cursor.release(); d_own.release();
+    if (tri_path) {
+        DRESS_CUDA_TRY(counted_memcpy(&T, d_ioff.get() + E, sizeof(T), cudaMemcpyDeviceToHost, st));
+        DRESS_CUDA_TRY(counted_memcpy(&listed, tri.total, sizeof(listed), cudaMemcpyDeviceToHost, st));
+        DRESS_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    if (E - e0 > 0) {
+    DRESS_TRY(d_pairs.alloc((size_t)(T > 0 ? T : 1), st));
+    if (tri_path && T > 0) {
+        DevBuf<unsigned long long> d_cursor;
+        DRESS_TRY(d_cursor.alloc((size_t)E, st));
+        DRESS_CUDA_TRY(cudaMemcpyAsync(d_cursor.get(), d_ioff.get(), (size_t)E * sizeof(long long),
+                                       cudaMemcpyDeviceToDevice, st));
+        if (!by_owner) count_launch(), k_renumber<<<tg, 256, 0, st>>>((int)M, d_einv.get(), d_oeid.get());
+        if ((long long)listed <= tri.cap)
+            count_launch(), k_triangle_pairs<<<grid_for((long long)listed, 256, 64 * sms), 256, 0, st>>>(
+                tri, d_oeid.get(), d_cursor.get(), d_pairs.get());
+        else
+            count_launch(), k_triangles<true><<<tg, 256, 0, st>>>((int)M, d_ooff.get(), d_otgt.get(), d_oeid.get(),
+                                                                  d_osrc.get(), nullptr, tri, d_cursor.get(),
+                                                                  d_pairs.get());
+    }
+    d_otgt.release(); d_oeid.release(); d_osrc.release(); d_ooff.release(); d_ocnt.release();
+    d_cntq.release(); d_tri.release();
+    if (!tri_path && E - e0 > 0) {
         const int c1 = ec.cls[1], c6 = ec.cls[6];
         if (c1 > 0)
             count_launch(), k_new_pairs<1><<<grid_for(c1, 256, 64 * sms), 256, 0, st>>>(
@@ -1139,8 +1364,27 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
                 L, c4, c5, d_ioff.get(), d_pairs.get());
         DRESS_CUDA_TRY(cudaGetLastError());
     }
-    d_U.release(); d_V.release(); d_w.release(); d_d.release(); d_nw.release();
     d_ioff_old.release(); d_ncnt.release(); d_cnt.release(); d_deg.release();
+
+    // The edge arrays in the new numbering.  Nothing above reads them when the
+    // triangle listing made the pairs, so all of it runs beside their upload
+    // (28 M edges: the set-up ends 33 ms after the call began, 44 when the
+    // renumbering waited for the edge arrays).
+    if (!edges_valid) DRESS_TRY(validate_edges());
+    DRESS_TRY(d_nwi.alloc((size_t)N, st));
+    DRESS_TRY(d_eu.alloc((size_t)E, st));
+    DRESS_TRY(d_ev.alloc((size_t)E, st));
+    DRESS_TRY(d_dbuf.alloc(2 * (size_t)E, st));
+    if (!uniform) {
+        DRESS_TRY(d_wi.alloc((size_t)E, st));
+        DRESS_TRY(d_pbuf.alloc(2 * (size_t)E, st));
+    }
+    count_launch(), k_new_nw<<<vg, 256, 0, st>>>(N, d_vperm.get(), d_nw.get(), d_nwi.get());
+    count_launch(), k_new_edges<<<eg, 256, 0, st>>>(E, d_eperm.get(), d_rec.get(), d_vinv.get(), d_eu.get(), d_ev.get(),
+                                    uniform ? nullptr : d_wi.get(), d_dbuf.get(),
+                                    uniform ? nullptr : d_pbuf.get());
+    DRESS_CUDA_TRY(cudaGetLastError());
+    d_U.release(); d_V.release(); d_w.release(); d_d.release(); d_nw.release(); d_rec.release();
 
     // exact sums of queued items: shared memory for their terms, a global
     // scratch slice per block for items beyond it
@@ -1349,8 +1593,8 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         stats->iterate_ms = sweep_ms;
         stats->phase_ms[0] = t_upload + edge_up.wait_ms;
         stats->phase_ms[1] = t_valid;
-        stats->phase_ms[2] = t_pairs - t_upload - edge_up.wait_ms - t_valid;
-        stats->phase_ms[3] = setup_ms - t_pairs;
+        stats->phase_ms[2] = t_pairs - t_upload - early_ms;
+        stats->phase_ms[3] = setup_ms - t_pairs - (edge_up.wait_ms + t_valid - early_ms);
         stats->phase_ms[4] = ms_since(t_down0);
     }
     return Status::Ok();

@@ -82,3 +82,29 @@ def test_out_of_range_on_the_way(variant, spread, iterations, oracle_port):
     W = np.exp(rng.uniform(-spread, spread, 5003))
     NW = rng.uniform(0.3, 5.0, n)
     _fit(oracle_port, n, U, V, W, NW, variant, max_iterations=iterations)
+
+
+@pytest.mark.parametrize("loops", [0, 3])
+def test_large_renumbering(loops, oracle_port):
+    """2^20 edges and more are renumbered by owner from the oriented rows, with
+    a self loop (which is in none) by sorted keys; rows of 1 to 1,500 slots."""
+    n, U, V = graphs.chung_lu(150_001, (1 << 20) + 5, 2.3, 1500, seed=4)
+    V[:loops] = U[:loops]
+    _fit(oracle_port, n, U, V, np.random.default_rng(5).uniform(0.5, 2.0, len(U)), max_iterations=4)
+
+
+@pytest.mark.parametrize("low", [2, 31, 32, 33, 511, 512, 513, 700])
+def test_owner_rows(low, oracle_port):
+    """A vertex whose oriented row has `low` members (hashed up to 512, then
+    searched), all of them of higher degree and some joined to each other."""
+    rng = np.random.default_rng(low)
+    core = np.arange(1, low + 1)
+    far = np.arange(low + 1, 2 * low + 41)
+    e = [np.stack([np.zeros(low, int), core], 1)]
+    e += [np.stack([np.full(low + 1, c), rng.choice(far, low + 1, replace=False)], 1) for c in core]
+    for _ in range(2):
+        e.append(np.stack([core, rng.permutation(core)], 1))
+    e = np.concatenate(e)
+    e = np.unique(np.sort(e[e[:, 0] != e[:, 1]], axis=1), axis=0)
+    e = e[rng.permutation(len(e))].astype(np.int32)
+    _fit(oracle_port, int(e.max()) + 1, e[:, 0].copy(), e[:, 1].copy(), max_iterations=5)
