@@ -88,8 +88,8 @@ struct Sweep {
 };
 
 // Per-sweep max|delta| slots form a ring; the sweep index lives in device
-// memory, so every sweep of a chunk is the same launch sequence (replayed from
-// a CUDA graph) and the sweeps after convergence return at once.
+// memory, so every sweep of a chunk is the same launch sequence (certified ones
+// are replayed from a CUDA graph) and the sweeps after convergence return at once.
 constexpr int RING = 64;
 
 __device__ __forceinline__ bool skipped(const Sweep &s)
