@@ -57,14 +57,14 @@ for _p in (ROOT, PKG):
 
 HBM_FALLBACK_GBS = 6650.0
 
-# k_batch on the 2,000-graph headline batch (64 threads per subgraph, two CTAs
+# k_batch on the 2,000-graph headline batch (32 threads per subgraph, two CTAs
 # per SM), one launch under `ncu --set full` (profiles/k_batch_delta1_2000graphs.md):
 # dram__bytes_read.sum + dram__bytes_write.sum, and the issue-bound figures
-KBATCH_HEADLINE_NCU = {"dram_bytes": 19.33e6 + 190.33e6,
-                       "issue": {"issue_active_frac": 0.724, "lanes_per_inst": 19.5, "fp64_pipe_frac": 0.227}}
+KBATCH_HEADLINE_NCU = {"dram_bytes": 10.11e6 + 182.36e6,
+                       "issue": {"issue_active_frac": 0.675, "lanes_per_inst": 28.1, "fp64_pipe_frac": 0.349}}
 
 # The 28M-edge single fit: dram__bytes_read.sum + dram__bytes_write.sum of the
-# twelve sweep kernels of one sweep (sweep 10), one capture per variant
+# two sweep kernels of one sweep (sweep 10), one capture per variant
 # (profiles/single_fit_chunglu28m_sweep_dram.md)
 SINGLE_FIT_NCU = {"edges": 28_000_000, "weighted": 4.218e9 + 0.512e9, "unweighted": 3.858e9 + 0.283e9}
 
