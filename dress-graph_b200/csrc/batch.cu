@@ -517,6 +517,10 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
         }
     }
 
+    // Without a sweep no barrier lies between the reads of ctl[0] and ctl[1] above
+    // and thread 0's reset of them below.
+    if (P.max_iter <= 0) g.sync();
+
     // ---- sweeps ------------------------------------------------------------------
     // Live products are positive on the fast path, so a zero marks a dead edge.
     const bool ones = P.kind == ITEM_DELTA || (P.kind == ITEM_PLAIN && !P.img.has_nw);   // every nw is 1.0

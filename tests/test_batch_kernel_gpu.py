@@ -112,3 +112,21 @@ def test_a_batch_of_every_size(oracle_port):
             np.testing.assert_array_equal(r[0], fn(*c, k=1, n_samples=12, seed=2)["hist"])
     for g in gs:
         g.close()
+
+
+@pytest.mark.parametrize("m,stride", [(20, 1), (33, 1), (200, 1), (1500, 40)])
+def test_no_sweeps(m, stride, oracle_port):
+    """max_iterations = 0: every live edge keeps its first value.  Groups of one
+    and of several warps, repeated so that warps of a group meet in any order."""
+    n, U, V = _sparse(max(14, m // 3), m, m)
+    W = np.random.default_rng(m).uniform(0.5, 2.0, m)
+    with db.Graph(n, U, V, W) as g:
+        for kind, fn in ((db.DELTA, oracle_port.delta_fit), (db.NABLA, oracle_port.nabla_fit)):
+            ref = fn(n, U, V, W, k=1, max_iterations=0, stride=stride)
+            for _ in range(5):
+                flat, _, _, fits, _ = db.hist_requests([g], kind, 1, max_iterations=0, stride=stride)[0]
+                np.testing.assert_array_equal(flat, ref["hist"])
+                assert flat.size and fits <= n
+        with db.Server() as srv:
+            r = srv.submit(g, db.DELTA, 1, max_iterations=0).wait()
+            np.testing.assert_array_equal(r["hist_flat"], oracle_port.delta_fit(n, U, V, W, k=1, max_iterations=0)["hist"])
