@@ -126,13 +126,15 @@ namespace {
 //     starts at 4 nw >= A, an edge sum at twice that (once, in the FORWARD and
 //     BACKWARD variants) and its terms are sums of two products;
 //   * at least PLO, a power of two with n a 2^-50 < PLO for the longest item's
-//     n terms and a bound a on any sum: every term, partial sum and rounding
-//     error is then a multiple of ulp(PLO) and every sum of errors is below
-//     2^53 of them, so the additions of errors are exact in any order.
+//     n terms and a bound a on any sum, and no larger than A, which no self term
+//     is below: every term, partial sum and rounding error is then a multiple of
+//     ulp(PLO) and every sum of errors is below 2^53 of them, so the additions of
+//     errors are exact in any order.
 // PHI is 4 nw rounded down to a power of two, doubled (unit weights: products
-// below 8), PLO about 2^-41 n^2: only products of zero or of values far from
+// below 8), PLO about 2^-45 n^2: only products of zero or of values far from
 // any fixed point are outside.  All in units of the weight where that is one
-// power of two.  span = 0: no fast path.
+// power of two.  span = 0: no fast path (vertex weights so far apart, or so far
+// below the edge weights, that PLO passes A).
 // w_max > 0: for the cluster fit, whose sums take terms of any size in any
 // order: PHI then only has to be above the products that occur.  Values stay
 // below about 2 sqrt(nw_max / nw_min); PHI is 16 to 32 times the largest weight
@@ -149,7 +151,7 @@ void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageSha
     const double n = most_terms;
     const double bound = 2.0 * Amax + 2.0 * (n + 1.0) * phi;
     const double plo = std::ldexp(1.0, std::ilogb(n * bound * 0x1p-50) + 1);
-    if (!(plo < phi)) return;
+    if (!(plo < phi) || !(plo <= A)) return;
     uint64_t b0, b1;
     std::memcpy(&b0, &plo, 8);
     std::memcpy(&b1, &phi, 8);

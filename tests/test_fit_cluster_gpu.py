@@ -73,3 +73,42 @@ def test_a_weight_out_of_range_goes_the_other_way(bad, oracle_port):
     W = np.random.default_rng(1).uniform(0.5, 2.0, 3000)
     W[1234] = bad
     _fit(oracle_port, n, U, V, W, one_launch=False)
+
+
+def rows_that_depend_on_the_order(first, count, seed):
+    """Weights of `count` rows whose sums after the term `first` are not the
+    sorted Neumaier sums when the rounding errors are added up in the order
+    given: `first` lies so far below the weights that the errors' sum loses it."""
+    w = np.random.default_rng(seed).uniform(32, 64, (40_000, 16))
+    x = np.concatenate([np.full((len(w), 1), first), w], axis=1)
+
+    def total(x):
+        s, c = x[:, 0].copy(), np.zeros(len(x))
+        for j in range(1, x.shape[1]):
+            t = s + x[:, j]
+            b = t - s
+            c = c + ((s - (t - b)) + (x[:, j] - b))
+            s = t
+        return np.sqrt(s + c)
+
+    rows = w[total(x) != total(np.sort(x, axis=1))]
+    assert len(rows) >= count
+    return rows[:count]
+
+
+@pytest.mark.parametrize("one_launch", [0, -1])
+def test_vertex_weights_far_below_the_products(one_launch, oracle_port):
+    """Self terms below the smallest product: errors are no multiples of its
+    last place, and only a certificate shows that a sum is the sorted one."""
+    first = 1.9 * 2.0 ** -97
+    w = rows_that_depend_on_the_order(first, 80, 3)
+    hub = np.arange(80)[:, None] * 17
+    U = np.broadcast_to(hub, (80, 16)).astype(np.int32).ravel()
+    V = (hub + np.arange(1, 17)).astype(np.int32).ravel()
+    db.configure(one_launch_max_edges=one_launch)
+    try:
+        for iterations in (1, 100):
+            _fit(oracle_port, 80 * 17, U, V, w.ravel(), np.full(80 * 17, first / 4), one_launch=None,
+                 max_iterations=iterations)
+    finally:
+        db.configure()
