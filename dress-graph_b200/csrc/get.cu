@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(256) k_get_sums(GetGraph G, long long n, const
             if (k < s1) {
                 const int x = G.tgt[k];
                 at = lower_bound(G.tgt, from, l1, x);
-                int r = 0;                             // place in a run of parallel edges
-                while (k - r > s0 && G.tgt[k - r - 1] == x) ++r;
-                if (r) at = lower_bound(G.tgt, G.off[b], l1, x);
-                if (at + r < l1 && G.tgt[at + r] == x) {
+                // place in a run of parallel edges, by search: a run of r would
+                // take r steps in each of its lanes
+                const int r = k > s0 && G.tgt[k - 1] == x ? k - lower_bound(G.tgt, s0, k, x) : 0;
+                if (r < l1 - at && G.tgt[at + r] == x) {
                     q.add(term_of(G, G.eidx[k], G.eidx[at + r]));
                     ++terms;
                 }

@@ -66,3 +66,14 @@ def test_power_law_pairs(exact, oracle_port):
     rng = np.random.default_rng(5)
     q = list(zip(rng.integers(0, n, 300).tolist(), rng.integers(0, n, 300).tolist()))
     _check(oracle_port, n, U, V, None, q)
+
+
+@pytest.mark.parametrize("run,other", [(31, 33), (64, 40), (1000, 999), (4000, 4100)])
+def test_long_runs_of_parallel_edges(run, other, oracle_port):
+    """Runs within, across and far beyond a warp's strip, of unequal length in
+    the two rows; the place in a run is found by search, not step by step."""
+    rng = np.random.default_rng(run)
+    U = np.concatenate([np.zeros(3 * run), np.ones(3 * other), [0, 1]]).astype(np.int32)
+    V = np.concatenate([np.repeat([2, 3, 5], run), np.repeat([2, 4, 5], other), [6, 6]]).astype(np.int32)
+    p = rng.permutation(len(U))
+    _check(oracle_port, 7, U[p], V[p], rng.uniform(0.5, 2.0, len(U)), [(0, 1), (1, 0), (2, 6), (0, 6)])
