@@ -3,6 +3,7 @@ synthetic measurements: the single-fit HBM fractions with the measured DRAM
 traffic, the serving percentiles and the other workloads' summaries stay on
 the one JSON line; full figures go to --detail.  CPU only."""
 import json
+import types
 
 import bench
 
@@ -48,3 +49,12 @@ def test_single_fit_traffic_constants_cover_both_variants():
     c = bench.SINGLE_FIT_NCU
     assert c["edges"] == 28_000_000
     assert 4e9 < c["unweighted"] < c["weighted"] < 6e9
+
+
+def test_no_reference_arm_without_the_reference(monkeypatch, capsys):
+    """Without the reference library the arm says so and times nothing."""
+    import oracle
+    monkeypatch.setattr(oracle, "reference", lambda: None)
+    bench.reference_arm(types.SimpleNamespace(graphs=2, warmup=0, steps=1, gpus=1), 0)
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
