@@ -86,3 +86,17 @@ def test_large_graph_layout_sorted_path(oracle_port, exact_sums):
     n, U, V = graphs.chung_lu(200_000, 1_200_000, 2.3, 3000, seed=5)
     W = graphs.uniform_weights(len(U), seed=6)
     assert_same(gpu_fit(n, U, V, W, max_iterations=4), oracle_port.fit(n, U, V, W, precompute=1, max_iterations=4))
+
+
+@pytest.mark.parametrize("n,m", [(30, 100), (60, 900), (5000, 30001)])
+def test_zero_weights_among_others(n, m, oracle_port):
+    """Zero terms in most sums, of which many are ties between two doubles."""
+    n, U, V = graphs.erdos_renyi(n, m, seed=m)
+    W = np.random.default_rng(m).integers(0, 4, m).astype(float)
+    W[::5] = -0.0
+    ref = oracle_port.fit(n, U, V, W)
+    with db.Graph(n, U, V, W) as g:
+        it, delta = db.fit_graph(g)
+        assert (it, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+        np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
