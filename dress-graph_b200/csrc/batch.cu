@@ -255,12 +255,24 @@ __device__ __forceinline__ State state_at(unsigned b, int E, int N, int k)
 // (libdress/src/dress.c:51-66) without a certificate per item: the "exact
 // compensation" case of CSum (common.cuh), decided once a sweep for all items.
 // Four additions a term; CSum takes eight FP64 operations and eight selects.
+// WIDE: TwoSum, six additions a term, which needs no order of the exponents, so
+// the range may reach above the running sums: products of 8 and more (edge
+// weights of 4 and more, vertex weights below 1).  Such parents took the slow
+// sums otherwise: a whole-graph fit of 300 edges with weights 1 to 10 228 us,
+// 163 so; the Delta^1 kernel of 60 graphs of 16 to 100 vertices with them 787 us,
+// 387 so (166 by the narrow sums at weights of 0.5 to 2).
+template <bool WIDE>
 struct FastSum {
     double s, c;
     __device__ __forceinline__ void add(double x)
     {
         const double t = dadd(s, x);
-        c = dadd(c, dsub(x, dsub(t, s)));
+        if (WIDE) {
+            const double b = dsub(t, s);
+            c = dadd(c, dadd(dsub(s, dsub(t, b)), dsub(x, b)));
+        } else {
+            c = dadd(c, dsub(x, dsub(t, s)));
+        }
         s = t;
     }
 };
@@ -448,12 +460,15 @@ __device__ __forceinline__ double term(const SArr<double> x, const ImageView<A> 
     return v != 0.0 ? dmul(G.w[i], v) : 0.0;       // the padding id has no weight
 }
 
-// One subgraph.  FAST: by FastSum; false, with nothing emitted, when a live
-// product leaves the fast range.  Otherwise every sum by item_sum.
-template <int MODE, template <class> class A, bool FAST>
+// One subgraph.  SUM_NARROW, SUM_WIDE: by FastSum; false, with nothing emitted,
+// when a live product leaves the range.  SUM_SLOW: every sum by item_sum.
+enum { SUM_NARROW = 0, SUM_WIDE = 1, SUM_SLOW = 2 };
+template <int MODE, template <class> class A, int SUM>
 __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A> &G, long long item, const Group &g,
                                          unsigned mem)
 {
+    constexpr bool FAST = SUM != SUM_SLOW;
+    using RangeSum = FastSum<SUM == SUM_WIDE>;
     const State st = state_at<MODE>(mem, P.E, P.N, P.k);
     unsigned *ctl = st.ctl.ptr();
     SArr<double> x0 = st.x0, x1 = st.x1;
@@ -500,7 +515,8 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
                 x0.set(e, al ? (MODE == STATE_PRODUCT ? p : d) : 0.0);
                 if (!al) x1.set(e, 0.0);
                 if (MODE == STATE_PRODUCT) st.dv.set(e, d);
-                out |= al && !in_range(p, P.img.lo, P.img.span);
+                out |= al && !in_range(p, SUM == SUM_WIDE ? P.img.wide_lo : P.img.lo,
+                                       SUM == SUM_WIDE ? P.img.wide_span : P.img.span);
             }
             const unsigned word = __ballot_sync(0xffffffffu, al);
             if ((g.t & 31) == 0) st.eb.ptr()[b0 >> 5] = word;
@@ -525,7 +541,7 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
     // Live products are positive on the fast path, so a zero marks a dead edge.
     const bool ones = P.kind == ITEM_DELTA || (P.kind == ITEM_PLAIN && !P.img.has_nw);   // every nw is 1.0
     const bool fwd = P.fwd != 0, plain = P.kind == ITEM_PLAIN;
-    const unsigned lo = P.img.lo, span = P.img.span;
+    const unsigned lo = SUM == SUM_WIDE ? P.img.wide_lo : P.img.lo, span = SUM == SUM_WIDE ? P.img.wide_span : P.img.span;
     const double eps = P.eps;
     const int N = P.N, E = P.E;
     int it = 0;
@@ -533,7 +549,7 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
     for (; it < P.max_iter; ++it) {
         if (FAST) {
             for (int u = g.t; u < N; u += g.size) {
-                FastSum q{ones ? base4 : four_nw(P, st, G, base4, u), 0.0};
+                RangeSum q{ones ? base4 : four_nw(P, st, G, base4, u), 0.0};
                 const unsigned row = G.row[u];
                 for (unsigned b = row & 0xffffu, e = row >> 16; b < e; ++b) {
                     const Four f(G.eid[b]);
@@ -569,7 +585,7 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
                     s0 = four_nw(P, st, G, base4, u);
                     if (!fwd) s0 = dadd(s0, four_nw(P, st, G, base4, v));
                 }
-                FastSum q{dadd(s0, fwd ? own : dadd(own, own)), 0.0};      // 2 own is exact
+                RangeSum q{dadd(s0, fwd ? own : dadd(own, own)), 0.0};      // 2 own is exact
                 if (rec.y != NO_PAIRS) {
                     uint2 id;
                     unsigned b = rec.y;
@@ -668,13 +684,20 @@ __device__ __forceinline__ bool fit_item(const ParentDesc &P, const ImageView<A>
     return true;
 }
 
-// The same off the fast path, as a call of its own: what it needs in registers
-// does not weigh on the fast loops.
-template <int MODE, template <class> class A>
-__device__ __noinline__ void fit_item_slow(const ParentDesc &P, const ImageView<A> G, long long item, const Group g,
+// The same by the other sums, as calls of their own: what they need in registers
+// does not weigh on the narrow loops.
+template <int MODE, template <class> class A, int SUM>
+__device__ __noinline__ bool fit_item_call(const ParentDesc &P, const ImageView<A> G, long long item, const Group g,
                                            unsigned mem)
 {
-    fit_item<MODE, A, false>(P, G, item, g, mem);
+    return fit_item<MODE, A, SUM>(P, G, item, g, mem);
+}
+template <int MODE, template <class> class A>
+__device__ __noinline__ void fit_item_rest(const ParentDesc &P, const ImageView<A> G, long long item, const Group g,
+                                           unsigned mem)
+{
+    if (!P.force_exact && P.img.wide_span && fit_item_call<MODE, A, SUM_WIDE>(P, G, item, g, mem)) return;
+    fit_item_call<MODE, A, SUM_SLOW>(P, G, item, g, mem);
 }
 
 // Every group of the CTA takes subgraphs of the chunk until none is left.
@@ -699,8 +722,10 @@ __device__ __forceinline__ void fit_chunk(const ParentDesc &P, const Chunk &ch, 
             g.sync();
         }
         if (item >= ch.count) return;
-        if (P.force_exact || !fit_item<MODE, A, true>(P, G, ch.first + item, g, mem))
-            fit_item_slow<MODE, A>(P, G, ch.first + item, g, mem);
+        // the cheapest sums whose range the parent's first products are in, then
+        // what a product that leaves it on the way needs
+        if (P.force_exact || P.img.span == 0 || !fit_item<MODE, A, SUM_NARROW>(P, G, ch.first + item, g, mem))
+            fit_item_rest<MODE, A>(P, G, ch.first + item, g, mem);
     }
 }
 

@@ -81,7 +81,9 @@ struct ImageShape {
     int uniform = 0;             // every weight is the same power of two, wc
     int has_nw = 0, has_dinit = 0;
     double wc = 1.0;
-    unsigned lo = 0, span = 0;   // high words a live product may have on the fast path (fast_range)
+    // high words a live product may have on the fast path (fast_range), and on
+    // the wide one (batch kernel); span 0: not to be tried
+    unsigned lo = 0, span = 0, wide_lo = 0, wide_span = 0;
 };
 
 // Per-request statistics record written by the kernel.

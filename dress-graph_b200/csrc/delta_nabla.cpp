@@ -135,8 +135,9 @@ namespace {
 // any fixed point are outside.  All in units of the weight where that is one
 // power of two.  span = 0: no fast path (vertex weights so far apart, or so far
 // below the edge weights, that PLO passes A).
-// w_max > 0: for the cluster fit, whose sums take terms of any size in any
-// order: PHI then only has to be above the products that occur.  Values stay
+// w_max > 0: for sums that take terms of any size in any order (the cluster and
+// multi-kernel fits, the batch kernel's wide sums): PHI then only has to be
+// above the products that occur.  Values stay
 // below about 2 sqrt(nw_max / nw_min); PHI is 16 to 32 times the largest weight
 // times that root, and PLO follows from it.
 void fast_range(double nw_min, double nw_max, int most_terms, bool fwd, ImageShape &s, double w_max = 0.0)
@@ -214,7 +215,23 @@ ImageShape plan_image(p_dress_graph_t g, const std::vector<int> &ioff, int kind,
     double lo = 1.0, hi = 1.0;
     if (kind == ITEM_PLAIN && has_nw) weight_bounds(g, lo, hi);
     else if (kind == ITEM_NABLA && k > 0) hi = std::sqrt((double)std::max(53, 2 * k + 1));   // no marker is larger
-    fast_range(lo, hi, most, g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD, s);
+    const bool fwd = g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD;
+    double w_max = 0.0;
+    for (int e = 0; e < E; ++e) w_max = g->edge_weight[e] > w_max ? g->edge_weight[e] : w_max;
+    if (w_max > 0.0) {
+        fast_range(lo, hi, most, fwd, s, w_max);
+        s.wide_lo = s.lo;
+        s.wide_span = s.span;
+    }
+    fast_range(lo, hi, most, fwd, s);
+    // a range that the first products are not all in is not tried
+    for (int e = 0; e < E && (s.span || s.wide_span); ++e) {
+        const double d = has_dinit ? g->edge_dress[e] : 1.0, p = s.uniform ? d : g->edge_weight[e] * d;
+        uint64_t b;
+        std::memcpy(&b, &p, 8);
+        if ((unsigned)(b >> 32) - s.lo >= s.span) s.span = 0;
+        if ((unsigned)(b >> 32) - s.wide_lo >= s.wide_span) s.wide_span = 0;
+    }
     return s;
 }
 

@@ -130,3 +130,40 @@ def test_no_sweeps(m, stride, oracle_port):
         with db.Server() as srv:
             r = srv.submit(g, db.DELTA, 1, max_iterations=0).wait()
             np.testing.assert_array_equal(r["hist_flat"], oracle_port.delta_fit(n, U, V, W, k=1, max_iterations=0)["hist"])
+
+
+@pytest.mark.parametrize("weights", ["one to ten", "below four", "four", "one of five", "thousands", "growing"])
+@pytest.mark.parametrize("n,m", [(14, 31), (40, 200), (110, 5995), (3000, 9800)])
+def test_products_above_the_sums(n, m, weights, oracle_port):
+    """Products that the four-addition sums do not take: at the edge of their
+    range, far above it, in one edge only, and growing past it sweep by sweep,
+    for every form of a subgraph's state."""
+    rng = np.random.default_rng(m)
+    n, U, V = graphs.erdos_renyi(n, m, seed=m)
+    W = {"one to ten": rng.integers(1, 11, m).astype(float), "below four": rng.uniform(3.9, 4.0, m),
+         "four": np.full(m, 4.0), "one of five": np.where(np.arange(m) == m // 2, 5.0, rng.uniform(0.5, 2.0, m)),
+         "thousands": rng.uniform(1.0, 5000.0, m), "growing": np.exp(rng.uniform(-4.0, 2.0, m))}[weights]
+    variant = [db.UNDIRECTED, db.FORWARD, db.BACKWARD][m % 3] if weights != "growing" else db.FORWARD
+    with db.Graph(n, U, V, W, variant=variant) as g:
+        _same(g, (n, U, V, W, variant), oracle_port, db.DELTA, 1, n_samples=4, seed=1)
+        _same(g, (n, U, V, W, variant), oracle_port, db.NABLA, 1, n_samples=4, seed=2)
+
+
+@pytest.mark.parametrize("m", [31, 300, 1023, 1024])
+@pytest.mark.parametrize("lo,hi", [(0.05, 0.1), (0.2, 1.0), (0.6, 40.0), (1e-4, 1.0)])
+def test_plain_fits_with_vertex_weights(m, lo, hi, oracle_port):
+    """Vertex weights below 1 and far apart, up to the most edges of one CTA; a
+    fit that goes on from values of its own."""
+    rng = np.random.default_rng(m)
+    n, U, V = _sparse(max(14, m // 3), m, m)
+    W = rng.uniform(0.5, 2.0, m) if m % 2 else None
+    NW = rng.uniform(lo, hi, n)
+    ref = oracle_port.fit(n, U, V, W, NW)
+    with db.Graph(n, U, V, W, NW) as g:
+        db.counters(reset=True)
+        db.fit_graph(g, 3, 0.0)
+        it, delta = db.fit_graph(g)
+        assert db.counters()["launches"] == 2
+        assert (it + 3, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+        np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
