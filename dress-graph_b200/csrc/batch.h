@@ -193,7 +193,8 @@ struct ClusterFit {
     double eps;
     ImageShape img;
     const unsigned char *data;           // cluster_layout
-    unsigned *pairs, *cursor;            // room for sum_e min(deg u, deg v) words; zero
+    unsigned *pairs, *cursor;            // room for 2 E + sum_e min(deg u, deg v) words, 8-byte aligned; zero
+    int certified;                       // sums with certificates; 0: within img's range
     double *values;                      // E final edge values, then N vertex norms
     unsigned long long *stats;           // ST_FITS 0: a product left the range, nothing was fitted
 };

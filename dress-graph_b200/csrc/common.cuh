@@ -9,6 +9,7 @@
 //     (CSum below) or, where the certificate fails, that sorted sum itself;
 //   * sqrt and division are the IEEE round-to-nearest forms.
 #pragma once
+#include <climits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -138,6 +139,64 @@ struct CSum {
         return false;
     }
 };
+
+// The exact sorted KBN of the self term (index cnt) and the live stored
+// terms, visited in ascending (value, index) order by repeated scans: no
+// storage, O(cnt^2) term evaluations.  Equal values are interchangeable in
+// the sum, so this is the reference's "sort, then KBN" (dress.c:51-66).  It
+// runs only for the items whose certified sum fails (about one in 1e9).
+template <class Terms>
+__device__ __noinline__ double sorted_sum_select(double self, int cnt, Terms term)
+{
+    double pv = -DRESS_INF, s = 0.0, c = 0.0;
+    int pj = -1;
+    bool first = true;
+    for (;;) {
+        double bv = DRESS_INF;
+        int bj = INT_MAX;
+        for (int j = 0; j <= cnt; ++j) {
+            double t = self;
+            if (j < cnt && !term(j, t)) continue;
+            if (t != t) return t;                    // a NaN term makes the sum NaN in any order
+            const bool after = t > pv || (t == pv && j > pj);
+            const bool better = t < bv || (t == bv && j < bj);
+            if (after && better) {
+                bv = t;
+                bj = j;
+            }
+        }
+        if (bj == INT_MAX) break;
+        if (first) {
+            s = bv;
+            first = false;
+        } else {
+            kbn_step(s, c, bv);
+        }
+        pv = bv;
+        pj = bj;
+    }
+    return dadd(s, c);
+}
+
+// Sum of the self term and the live ones among cnt stored terms (term(j, t)
+// yields stored term j and whether it is alive): a certified sum in stored
+// order (CSum, common.cuh), the exact sorted sum where the certificate fails.
+template <class Terms>
+__device__ __forceinline__ double item_sum(double self, int cnt, const Terms &term, bool force_exact)
+{
+    if (cnt == 0) return dadd(self, 0.0);        // one term: the reference's sum + comp
+    if (force_exact) return sorted_sum_select(self, cnt, term);
+    CSum q;
+    q.init();
+    q.add(self);
+    for (int j = 0; j < cnt; ++j) {
+        double t;
+        if (term(j, t)) q.add(t);
+    }
+    double r;
+    if (q.result(r)) return r;
+    return sorted_sum_select(self, cnt, term);
+}
 
 // Cooperative in-place ascending sort of buf[0..n) by `nthr` threads with
 // index `tid` (a warp or a whole block).  Same single-direction bitonic

@@ -248,17 +248,26 @@ ImageShape plan_cluster(p_dress_graph_t g, int max_deg)
     const int E = g->E;
     s.Q = g->adj_offset[g->N];
     uniform_weight(g, s);
-    double lo, hi, w_max = 0.0;
+    double lo, hi, w_max = 0.0, w_min = HUGE_VAL;
     weight_bounds(g, lo, hi);
     s.has_nw = g->NW && !(lo == 1.0 && hi == 1.0);
     for (int e = 0; e < E; ++e) {
         s.has_dinit |= g->edge_dress[e] != 1.0;
         w_max = g->edge_weight[e] > w_max ? g->edge_weight[e] : w_max;
+        w_min = g->edge_weight[e] < w_min ? g->edge_weight[e] : w_min;
     }
     // a row's or an edge's terms, and the merges of its partial sums
     if (w_max > 0.0)
         fast_range(lo, hi, max_deg + 16, g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD, s,
                    w_max);
+    // first products that are the weights: a range that they are not in is not tried
+    if (!s.has_dinit)
+        for (double p : {w_min, w_max}) {
+            uint64_t b;
+            if (s.uniform) p = 1.0;
+            std::memcpy(&b, &p, 8);
+            if ((unsigned)(b >> 32) - s.lo >= s.span) s.span = 0;
+        }
     return s;
 }
 

@@ -21,11 +21,22 @@
 // (fast_range, delta_nabla.cpp), so a row's partial sums over several lanes
 // merge to the reference's bits.  TwoSum instead of Fast2Sum: a lane's partial
 // sum may start with its smallest term.  A product outside the range ends the
-// kernel with ST_FITS = 0, and the caller fits the graph another way.
+// kernel with ST_FITS = 0.
+//
+// Graphs whose products leave the range are fitted with a certificate per sum
+// (CERT: CSum, common.cuh), from the start, by the same kernel; another launch
+// over the whole device finds the pairs first, whose walks would otherwise be a
+// part of eight SMs' work.  (Going on from the sweep that left, instead, saved a
+// few microseconds and cost the uncertified kernel 4 to 8 % through its
+// registers.)  G(2000, 10000) with one weight of zero: 314 us a
+// call; 1,503 through the multi-kernel fit, 564 by an earlier certified cluster
+// kernel that gathered every term from its owner.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "batch.h"
 #include "common.cuh"
@@ -72,18 +83,26 @@ __device__ __forceinline__ void put_u32(unsigned a, unsigned v)
 // s + c = the exact sum so far (TwoSum; c is exact within the fast range)
 struct ExactSum {
     double s, c;
+    __device__ __forceinline__ void init() { s = c = 0.0; }
+    __device__ __forceinline__ void start(double x) { s = x; }
     __device__ __forceinline__ void add(double x)
     {
         const double t = dadd(s, x), b = dsub(t, s);
         c = dadd(c, dadd(dsub(s, dsub(t, b)), dsub(x, b)));
         s = t;
     }
-    __device__ __forceinline__ void merge(int o)
+    __device__ __forceinline__ void merge_lanes(int width)
     {
-        const double os = __shfl_xor_sync(0xffffffffu, s, o), oc = __shfl_xor_sync(0xffffffffu, c, o);
-        c = dadd(c, oc);
-        add(os);
+        for (int o = width >> 1; o > 0; o >>= 1) {
+            const double os = __shfl_xor_sync(0xffffffffu, s, o), oc = __shfl_xor_sync(0xffffffffu, c, o);
+            c = dadd(c, oc);
+            add(os);
+        }
     }
+    __device__ __forceinline__ double value() const { return dadd(s, c); }
+};
+struct CertSum : CSum {
+    __device__ __forceinline__ void start(double x) { add(x); }
 };
 
 struct Args {
@@ -93,10 +112,61 @@ struct Args {
     double eps;
     ImageShape img;
     const unsigned char *data;
-    unsigned *pairs, *cursor;                // room for every pair; words taken
+    unsigned *pairs, *cursor;                // room for every pair; words taken (CERT: edge_pairs first)
     double *values;
     unsigned long long *stats;
 };
+
+// CERT: every edge's first pair and their count, ahead of the pairs.  (In their
+// place rather than by a pointer of its own: 8 bytes more of arguments change the
+// other kernel's registers, and it took 3 % longer.)
+__device__ __forceinline__ uint2 *edge_pairs(const Args &A) { return (uint2 *)A.pairs; }
+template <bool CERT>
+__device__ __forceinline__ unsigned *all_pairs(const Args &A)
+{
+    return CERT ? A.pairs + 2 * A.E : A.pairs;
+}
+
+// CERT: the pairs of every edge, a thread each (the merge walk of the kernel below).
+constexpr int PAIR_THREADS = 64;
+__global__ void __launch_bounds__(PAIR_THREADS) k_cluster_pairs(const Args A)
+{
+    const ClusterLayout L = cluster_layout(A.N, A.E, A.img.Q, A.img.uniform, A.img.has_nw, A.img.has_dinit);
+    const unsigned short *off = (const unsigned short *)(A.data + L.off), *tgt = (const unsigned short *)(A.data + L.tgt);
+    const unsigned short *eid = (const unsigned short *)(A.data + L.eid);
+    const int e = blockIdx.x * PAIR_THREADS + threadIdx.x, lane = threadIdx.x & 31;
+    int iu0 = 0, iv0 = 0, iu_end = 0, iv_end = 0;
+    unsigned count = 0;
+    if (e < A.E) {
+        const unsigned uv = ((const unsigned *)(A.data + L.uv))[e], u = uv & 0xffffu, v = uv >> 16;
+        iu0 = off[u], iu_end = off[u + 1];
+        iv0 = off[v], iv_end = off[v + 1];
+        for (int iu = iu0, iv = iv0; iu < iu_end && iv < iv_end;) {
+            const unsigned x = tgt[iu], y = tgt[iv];
+            count += x == y;
+            iu += x <= y;
+            iv += x >= y;
+        }
+    }
+    unsigned at = count;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += y;
+    }
+    unsigned base = 0;
+    if (lane == 31 && at) base = atomicAdd(A.cursor, at);
+    at += __shfl_sync(0xffffffffu, base, 31) - count;
+    if (e >= A.E) return;
+    edge_pairs(A)[e] = make_uint2(at, count);
+    unsigned *pairs = all_pairs<true>(A);
+    const unsigned end = at + count;
+    for (int iu = iu0, iv = iv0; at < end;) {
+        const unsigned x = tgt[iu], y = tgt[iv];
+        if (x == y) pairs[at++] = (unsigned)eid[iu] | (unsigned)eid[iv] << 16;
+        iu += x <= y;
+        iv += x >= y;
+    }
+}
 
 // One CTA's shared memory: values (twice where they fit), norms; control words.
 struct Ctl {
@@ -105,6 +175,7 @@ struct Ctl {
     unsigned far[3], bad, part[33], base;
 };
 
+template <bool CERT>
 __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -120,22 +191,34 @@ __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
     const unsigned short *eid = (const unsigned short *)(A.data + L.eid);
     const double *w = (const double *)(A.data + L.w);
     const double *nw = A.img.has_nw ? (const double *)(A.data + L.nw) : nullptr;
-    const bool uni = A.img.uniform != 0;
+    const bool one_w = A.img.uniform != 0;
+    // sums in units of the weight where that is one power of two; certified sums
+    // take every product in full (units could over- or underflow)
+    const bool uni = one_w && !CERT;
     const int nv = (N + CTAS - 1) / CTAS, ne = (E + CTAS - 1) / CTAS;
     const int u0 = min(N, (int)rank * nv), u1 = min(N, u0 + nv), e0 = min(E, (int)rank * ne), e1 = min(E, e0 + ne);
     const double wc = A.img.wc, base4 = uni ? ddiv(4.0, wc) : 4.0;
 
     // ---- pairs of this thread's edges, by merge walks over staged rows -------------
     unsigned own_uv[OWN], first[OWN], count[OWN];
-    {
+    if (t == 0) {
+        ctl->bad = ctl->far[0] = ctl->far[1] = ctl->far[2] = 0;
+        ctl->largest = 0ULL;
+    }
+    if (CERT) {
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {
+            const int e = e0 + j * THREADS + t;
+            own_uv[j] = e < e1 ? uv[e] : 0u;
+            const uint2 r = e < e1 ? edge_pairs(A)[e] : make_uint2(0u, 0u);
+            first[j] = r.x;
+            count[j] = r.y;
+        }
+    } else {
         unsigned short *so = (unsigned short *)x0, *st = so + ((N + 2) & ~1);
         const unsigned short *tgt = (const unsigned short *)(A.data + L.tgt);
         for (int i = t; i <= N; i += THREADS) so[i] = off[i];
         for (int i = t; i < A.img.Q; i += THREADS) st[i] = tgt[i];
-        if (t == 0) {
-            ctl->bad = ctl->far[0] = ctl->far[1] = ctl->far[2] = 0;
-            ctl->largest = 0ULL;
-        }
         __syncthreads();
         unsigned mine = 0;
 #pragma unroll
@@ -212,9 +295,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
         bool out = false;
         for (int e = t; e < E; e += THREADS) {
             const double d = A.img.has_dinit ? dinit[e] : 1.0;
-            const double p = uni ? d : dmul(w[e], d);
+            const double p = uni ? d : dmul(CERT && one_w ? wc : w[e], d);
             x0[e] = p;
-            out |= (unsigned)__double2hiint(p) - A.img.lo >= A.img.span;
+            out |= !CERT && (unsigned)__double2hiint(p) - A.img.lo >= A.img.span;
         }
         if (__syncthreads_or(out)) {         // every CTA checks every value: all leave
             if (rank == 0 && t == 0) A.stats[ST_FITS] = 0ULL;
@@ -233,15 +316,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
     cluster_sync();                          // every CTA runs and has its copy
 
     // ---- sweeps ------------------------------------------------------------------------
+    using Sum = std::conditional_t<CERT, CertSum, ExactSum>;
     const int lpv = A.lpv, sub = t & (lpv - 1);
     int it = 0;
     double lmax = 0.0;
     for (; it < A.max_iter; ++it) {
         for (int b = u0; b < u1; b += THREADS / lpv) {
             const int u = b + t / lpv;
-            ExactSum q{0.0, 0.0};
+            Sum q;
+            q.init();
             if (u < u1) {
-                if (sub == 0) q.s = nw ? dmul(base4, nw[u]) : base4;
+                if (sub == 0) q.start(nw ? dmul(base4, nw[u]) : base4);
                 int k = off[u] + sub;
                 const int end = off[u + 1];
                 for (; k + 3 * lpv < end; k += 4 * lpv) {
@@ -259,9 +344,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
                 if (k + lpv < end) q.add(v1);
                 if (k + 2 * lpv < end) q.add(v2);
             }
-            for (int o = lpv >> 1; o > 0; o >>= 1) q.merge(o);
+            q.merge_lanes(lpv);
             if (u < u1) {
-                const double S = dadd(q.s, q.c);
+                double S;
+                if constexpr (CERT) {
+                    if (!q.result(S)) {      // every lane of the vertex
+                        const double *x = x0;
+                        const unsigned short *id = eid + off[u];
+                        S = sorted_sum_select(nw ? dmul(base4, nw[u]) : base4, off[u + 1] - off[u],
+                                              [=](int k, double &v) { return v = x[id[k]], true; });
+                    }
+                } else {
+                    S = q.value();
+                }
                 const double v = dsqrt(uni ? dmul(wc, S) : S);
                 if (A.spread) {
                     if (sub == 0) vd[u - u0] = v;
@@ -294,15 +389,30 @@ __global__ void __launch_bounds__(THREADS, 1) k_fit_cluster(const Args A)
                 const double den = dmul(nu, nn);
                 double s0 = nw ? dmul(base4, nw[u]) : base4;
                 if (!A.fwd) s0 = dadd(s0, nw ? dmul(base4, nw[v]) : base4);
-                ExactSum q{dadd(s0, A.fwd ? own : dadd(own, own)), 0.0};
+                const double self = dadd(s0, A.fwd ? own : dadd(own, own));
+                Sum q;
+                q.init();
+                q.start(self);
                 for (unsigned k = 0; k < count[j]; ++k) {
-                    const unsigned pr = A.pairs[first[j] + k];
+                    const unsigned pr = all_pairs<CERT>(A)[first[j] + k];
                     q.add(dadd(x0[pr & 0xffffu], x0[pr >> 16]));
                 }
-                const double S = dadd(q.s, q.c);
-                const double r = ddiv(uni ? dmul(wc, S) : S, den);
-                p[j] = uni ? r : dmul(w[e], r);
-                out |= (unsigned)__double2hiint(p[j]) - A.img.lo >= A.img.span;
+                double S;
+                if constexpr (CERT) {
+                    if (!q.result(S)) {
+                        const double *x = x0;
+                        const unsigned *pp = all_pairs<CERT>(A) + first[j];
+                        S = sorted_sum_select(self, (int)count[j], [=](int k, double &v) {
+                            return v = dadd(x[pp[k] & 0xffffu], x[pp[k] >> 16]), true;
+                        });
+                    }
+                } else {
+                    S = q.value();
+                }
+                double r = ddiv(uni ? dmul(wc, S) : S, den);
+                if (CERT) r = den > 0.0 ? r : 0.0;           // (positive in the range)
+                p[j] = uni ? r : dmul(CERT && one_w ? wc : w[e], r);
+                out |= !CERT && (unsigned)__double2hiint(p[j]) - A.img.lo >= A.img.span;
                 const double dd = fabs(dsub(val[j], r));
                 val[j] = r;
                 far |= dd >= A.eps;
@@ -432,21 +542,28 @@ Status launch_cluster_fit(const ClusterFit &f, cudaStream_t st)
         std::lock_guard<std::mutex> lk(mu);
         auto it = placeable.find(dev);
         if (it == placeable.end()) {
-            DRESS_CUDA_TRY(cudaFuncSetAttribute(k_fit_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)CLUSTER_SMEM));
-            int clusters = 0;
-            cfg.dynamicSmemBytes = CLUSTER_SMEM;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_fit_cluster, &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                clusters = 0;
+            int clusters = INT_MAX;
+            for (void (*k)(const Args) : {k_fit_cluster<false>, k_fit_cluster<true>}) {
+                DRESS_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM));
+                int n = 0;
+                cfg.dynamicSmemBytes = CLUSTER_SMEM;
+                if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+                    cudaGetLastError();
+                    n = 0;
+                }
+                clusters = std::min(clusters, n);
             }
             it = placeable.emplace(dev, clusters).first;
         }
         if (it->second < 1) return Status::Err(DRESSX_EUNSUPPORTED, "cluster fit does not fit the device");
     }
+    if (f.certified) {
+        count_launch(), k_cluster_pairs<<<(f.E + PAIR_THREADS - 1) / PAIR_THREADS, PAIR_THREADS, 0, st>>>(a);
+        DRESS_CUDA_TRY(cudaGetLastError());
+    }
     cfg.dynamicSmemBytes = smem;
     count_launch();
-    DRESS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_fit_cluster, a));
+    DRESS_CUDA_TRY(cudaLaunchKernelEx(&cfg, f.certified ? k_fit_cluster<true> : k_fit_cluster<false>, a));
     return Status::Ok();
 }
 

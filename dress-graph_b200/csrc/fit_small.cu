@@ -7,7 +7,7 @@
 // whole-graph item: every sweep, the convergence test and the final values in
 // one launch, without per-sweep kernels or host round trips.  Graphs of up to
 // CLUSTER_MAX_EDGES edges run on a thread-block cluster whose CTAs hold the
-// values each (fit_cluster.cu).  Larger graphs, and graphs that carry their own
+// values each (fit_cluster.cu), in two launches where products are out of range.  Larger graphs, and graphs that carry their own
 // intercept tables, take the multi-kernel fit in fit_graph.cu.  Bit-identical
 // to the reference all.
 #include <algorithm>
@@ -101,7 +101,6 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         image = image_layout(N, E, img.Q, img.P2, img.uniform, img.has_nw, 1).bytes;
     } else {
         img = plan_cluster(g, maxdeg);
-        if (img.span == 0) return Status::Ok();
         image = cluster_layout(N, E, img.Q, img.uniform, img.has_nw, img.has_dinit).bytes;
         T = 0;
         for (int e = 0; e < E; ++e)          // room for every pair
@@ -111,7 +110,7 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // One device block holds everything: the packed image, the descriptor, the
     // chunk, the counter, the statistics and the results (and a cluster's
-    // pairs).  The host writes the inputs once, into the context's pinned
+    // pairs and where each edge's begin).  The host writes the inputs once, into the context's pinned
     // stage, and one copy each way moves them.
     auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
     const size_t off_desc = al((size_t)image);
@@ -122,7 +121,8 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     const size_t total = off_vals + ((size_t)E + N) * sizeof(double);
     cudaStream_t st = ctx.st;
     DevBuf<unsigned char> d_blob;
-    DRESS_TRY(d_blob.alloc(al(total) + (one_cta ? 0 : 4 * (size_t)T), st));
+    const size_t off_pairs = al(total);
+    DRESS_TRY(d_blob.alloc(one_cta ? total : off_pairs + 8 * (size_t)E + 4 * (size_t)T, st));
     DRESS_TRY(ctx.stage->reserve(total));
     unsigned char *h = (unsigned char *)ctx.stage->ptr();
     unsigned char *dv = d_blob.get();
@@ -168,23 +168,32 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     } guard{e0, e1};
     const double setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     DRESS_CUDA_TRY(cudaEventRecord(e0, st));
-    if (one_cta) {
-        DRESS_TRY(launch_batch(L, ctx.num_sms, st));
-    } else {
-        const ClusterFit cf{N, E, fwd, max_iterations, epsilon, img, dv, (unsigned *)(dv + al(total)),
-                            (unsigned *)(dv + off_ctr), (double *)(dv + off_vals), (unsigned long long *)(dv + off_stats)};
-        Status ls = launch_cluster_fit(cf, st);
-        if (ls.code == DRESSX_EUNSUPPORTED) return Status::Ok();     // the multi-kernel fit takes it
-        DRESS_TRY(ls);
-    }
-    DRESS_CUDA_TRY(cudaEventRecord(e1, st));
-
-    // statistics and results come back in one copy through the stage
-    DRESS_CUDA_TRY(counted_memcpy(h + off_stats, dv + off_stats, total - off_stats, cudaMemcpyDeviceToHost, st));
-    DRESS_CUDA_TRY(cudaStreamSynchronize(st));
+    // A cluster sums within the range that the host knows the products to begin
+    // in; where they are outside, or leave it on the way, with certificates.
+    bool certified = img.span == 0;
     unsigned long long sv[ST_WORDS];
-    std::memcpy(sv, h + off_stats, sizeof sv);
-    if (sv[ST_FITS] == 0) return Status::Ok();       // a product left the cluster's range: the multi-kernel fit takes it
+    for (;;) {
+        if (one_cta) {
+            DRESS_TRY(launch_batch(L, ctx.num_sms, st));
+        } else {
+            const ClusterFit cf{N, E, fwd, max_iterations, epsilon, img, dv, (unsigned *)(dv + off_pairs),
+                                (unsigned *)(dv + off_ctr), certified, (double *)(dv + off_vals),
+                                (unsigned long long *)(dv + off_stats)};
+            Status ls = launch_cluster_fit(cf, st);
+            if (ls.code == DRESSX_EUNSUPPORTED) return Status::Ok();     // the multi-kernel fit takes it
+            DRESS_TRY(ls);
+        }
+        DRESS_CUDA_TRY(cudaEventRecord(e1, st));
+
+        // statistics and results come back in one copy through the stage
+        DRESS_CUDA_TRY(counted_memcpy(h + off_stats, dv + off_stats, total - off_stats, cudaMemcpyDeviceToHost, st));
+        DRESS_CUDA_TRY(cudaStreamSynchronize(st));
+        std::memcpy(sv, h + off_stats, sizeof sv);
+        if (sv[ST_FITS] != 0) break;
+        if (one_cta || certified) return Status::Ok();               // (neither gives up)
+        certified = true;
+        DRESS_CUDA_TRY(cudaMemsetAsync(dv + off_ctr, 0, sizeof(int), st));
+    }
     std::memcpy(g->edge_dress, h + off_vals, (size_t)E * sizeof(double));
     // the norms of the last sweep (none without sweeps), as fit_graph leaves them
     if (sv[ST_SWEEPS] > 0) std::memcpy(g->vertex_dress, h + off_vals + (size_t)E * sizeof(double), (size_t)N * sizeof(double));

@@ -2,6 +2,8 @@
 bit for bit against the oracle: one and two value buffers, one to eight lanes a
 vertex, edges a thread owns one to four of, variants, vertex weights, values to
 go on from, and weights that take the fit off this path."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -112,3 +114,81 @@ def test_vertex_weights_far_below_the_products(one_launch, oracle_port):
                  max_iterations=iterations)
     finally:
         db.configure()
+
+
+def _certified(oracle_port, launches, *case, **kw):
+    """_fit's comparison for fits that take `launches`: the pairs and certified
+    sweeps, after an attempt within the range where that only shows on the way."""
+    ref = oracle_port.fit(*case, **kw)
+    variant = kw.pop("variant", db.UNDIRECTED)
+    with db.Graph(*case, variant) as g:
+        db.counters(reset=True)
+        it, delta = db.fit_graph(g, **kw)
+        assert launches is None or db.counters()["launches"] == launches
+        assert (it, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+        np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
+
+
+@pytest.mark.parametrize("n,m", [(500, 1025), (700, 2049), (2000, 10000), (120, 4000), (9000, 16385), (400, 24001),
+                                 (8000, 22000), (16000, 24575)])
+@pytest.mark.parametrize("weights", ["one zero", "zeros", "signed", "tiny", "halves of zero vertices"])
+def test_certified_sizes(n, m, weights, oracle_port):
+    """The shapes of test_sizes off the range, in two launches."""
+    n, U, V = graphs.erdos_renyi(n, m, seed=m)
+    rng = np.random.default_rng(m)
+    W = rng.uniform(0.5, 2.0, m)
+    NW = None
+    if weights == "one zero":
+        W[m // 2] = 0.0
+    elif weights == "zeros":
+        W = rng.integers(0, 4, m).astype(float)
+    elif weights == "signed":
+        W = np.where(rng.random(m) < 0.05, -0.01, W)
+    elif weights == "tiny":
+        W[::3] = 1e-305
+    else:
+        W, NW = np.full(m, 0.5), rng.integers(0, 2, n).astype(float)
+    _certified(oracle_port, 2, n, U, V, W, NW)
+
+
+@pytest.mark.parametrize("variant", [db.UNDIRECTED, db.DIRECTED, db.FORWARD, db.BACKWARD])
+@pytest.mark.parametrize("iterations", [1, 2, 3, 100])
+def test_certified_variants_and_sweep_limits(variant, iterations, oracle_port):
+    n, U, V = graphs.erdos_renyi(900, 5003, seed=7)
+    rng = np.random.default_rng(variant)
+    W = np.where(rng.random(5003) < 0.1, 0.0, rng.uniform(0.5, 2.0, 5003))
+    _certified(oracle_port, 2, n, U, V, W, rng.uniform(0.3, 5.0, n), variant=variant, max_iterations=iterations)
+    _certified(oracle_port, 2, n, U, V, W, None, variant=variant, max_iterations=iterations, epsilon=0.0)
+
+
+@pytest.mark.parametrize("spread", [6.0, 7.0, 8.0])
+def test_out_of_range_on_the_way(spread, oracle_port):
+    """FORWARD rows with weights over many binades grow past the range."""
+    n, U, V = graphs.erdos_renyi(900, 5003, seed=7)
+    rng = np.random.default_rng(int(spread * 10))
+    W = np.exp(rng.uniform(-spread, spread, 5003))
+    NW = rng.uniform(0.3, 5.0, n)
+    for kw in ({}, dict(epsilon=0.0), dict(max_iterations=60), dict(max_iterations=61)):
+        _certified(oracle_port, 3, n, U, V, W, NW, variant=db.FORWARD, **kw)
+    # up to the last sweep in range and past it, one launch and three
+    for iterations in range(1, 40):
+        _certified(oracle_port, None, n, U, V, W, NW, variant=db.FORWARD, max_iterations=iterations)
+
+
+def test_values_out_of_range_to_go_on_from(oracle_port):
+    """First values that put a product outside, which the host does not look for."""
+    n, U, V = graphs.erdos_renyi(900, 5003, seed=7)
+    d = np.ones(5003)
+    d[17] = 1e-200
+    ref = oracle_port.build(n, U, V)
+    ctypes.memmove(ref.contents.edge_dress, d.ctypes.data, d.nbytes)
+    it, delta = ctypes.c_int(), ctypes.c_double()
+    oracle_port.fit_fn(ref, 100, 1e-6, ctypes.byref(it), ctypes.byref(delta))
+    with db.Graph(n, U, V) as g:
+        ctypes.memmove(g.ptr.contents.edge_dress, d.ctypes.data, d.nbytes)
+        db.counters(reset=True)
+        assert db.fit_graph(g) == (it.value, delta.value)
+        assert db.counters()["launches"] == 3
+        want = np.ctypeslib.as_array(ref.contents.edge_dress, shape=(5003,))
+        np.testing.assert_array_equal(g.edge_dress.view(np.int64), want.view(np.int64))
