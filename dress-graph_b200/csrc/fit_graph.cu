@@ -59,7 +59,9 @@ __device__ __forceinline__ unsigned lanemask_lt()
 // flags[2]: edge weights are not all bit-identical, flags[3]: max row length,
 // flags[4..5]: the largest positive weight (bits of the double), flags[6]: an
 // edge id stands in two oriented slots (k_slot_counts), flags[8..11]:
-// the smallest and largest vertex weight (k_nw_bounds).
+// the smallest and largest vertex weight (k_nw_bounds), flags[12..13]: the
+// complement of the smallest and the largest high word of the first products
+// w*d that are not zero.
 // One warp per row (a hub's row is spread over the lanes).  A row outside
 // [0, S) or with end < begin is flagged and not read, so a malformed
 // adj_offset never leads to a read outside adj_target.
@@ -110,17 +112,43 @@ __global__ void k_validate_edges(int N, int E, const int *__restrict__ U, const 
 {
     unsigned long long w0 = E > 0 ? (unsigned long long)__double_as_longlong(w[0]) : 0ULL;
     double wm = 0.0;
+    unsigned not_lo = 0, hi = 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
         int u = U[e], v = V[e];
         if (u < 0 || u >= N || v < 0 || v >= N) atomicOr(&flags[0], 8);
-        const double we = w[e];
-        rec[e] = EdgeRec{u, v, we, d[e], 0.0};
+        const double we = w[e], de = d[e], p = dmul(we, de);
+        rec[e] = EdgeRec{u, v, we, de, 0.0};
         if ((unsigned long long)__double_as_longlong(we) != w0) flags[2] = 1;
         wm = we > wm ? we : wm;
+        if (p != 0.0) {
+            not_lo = max(not_lo, ~(unsigned)__double2hiint(p));
+            hi = max(hi, (unsigned)__double2hiint(p));
+        }
     }
+    // one atomic a block: thousands of warps on one word took 250 us
+    __shared__ double bw[8];
+    __shared__ unsigned bl[8], bh[8];
     for (int o = 16; o > 0; o >>= 1) wm = fmax(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-    if ((threadIdx.x & 31) == 0 && wm > 0.0)
-        atomicMax((unsigned long long *)(flags + 4), (unsigned long long)__double_as_longlong(wm));
+    not_lo = __reduce_max_sync(0xffffffffu, not_lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;      // 256 threads
+    if (lane == 0) {
+        bw[warp] = wm;
+        bl[warp] = not_lo;
+        bh[warp] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < warps; ++i) {
+            wm = fmax(wm, bw[i]);
+            not_lo = max(not_lo, bl[i]);
+            hi = max(hi, bh[i]);
+        }
+        if (wm > 0.0)
+            atomicMax((unsigned long long *)(flags + 4), (unsigned long long)__double_as_longlong(wm));
+        atomicMax((unsigned *)flags + 12, not_lo);
+        atomicMax((unsigned *)flags + 13, hi);
+    }
 }
 
 // Smallest and largest vertex weight as bits of positive doubles; a weight that
@@ -1006,15 +1034,16 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // ---- validate the rows ---------------------------------------------------
     DevBuf<int> d_flags, d_deg, d_cnt;
-    DRESS_TRY(d_flags.alloc(12, st));
+    constexpr int NFLAGS = 14;
+    DRESS_TRY(d_flags.alloc(NFLAGS, st));
     DRESS_TRY(d_deg.alloc((size_t)N, st));
     DRESS_TRY(d_cnt.alloc((size_t)E, st));
-    DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get(), 0, 12 * sizeof(int), st));
+    DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get(), 0, NFLAGS * sizeof(int), st));
     DRESS_CUDA_TRY(cudaMemsetAsync(d_flags.get() + 8, 0xff, 2 * sizeof(int), st));
     count_launch(), k_validate_rows<<<grid_for((long long)N * 32, 256, 16 * sms), 256, 0, st>>>(
         N, E, S, d_off.get(), d_tgt.get(), d_eidx.get(), d_deg.get(), d_flags.get());
     DRESS_CUDA_TRY(cudaGetLastError());
-    int flags[12];
+    int flags[NFLAGS];
     DRESS_CUDA_TRY(counted_memcpy(flags, d_flags.get(), sizeof(flags), cudaMemcpyDeviceToHost, st));
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));
     double t_valid = ms_since(t0) - t_upload;
@@ -1026,6 +1055,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     // pairs unless the triangle listing (CSR only) makes them.
     bool uniform = true;
     double w_max = 0.0, nw_lo = 1.0, nw_hi = 1.0;      // NULL vertex weights mean all 1.0
+    unsigned p_lo = 0, p_hi = 0;                       // high words of the first products
     bool edges_valid = false;
     DevBuf<EdgeRec> d_rec;
     auto validate_edges = [&]() -> Status {
@@ -1046,6 +1076,8 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         edges_valid = true;
         uniform = flags[2] == 0;
         std::memcpy(&w_max, flags + 4, sizeof w_max);
+        p_lo = ~(unsigned)flags[12];
+        p_hi = (unsigned)flags[13];
         if (g->NW && N) {
             std::memcpy(&nw_lo, flags + 8, sizeof nw_lo);
             std::memcpy(&nw_hi, flags + 10, sizeof nw_hi);
@@ -1477,7 +1509,8 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     const ImageShape range = plan_products(nw_lo, nw_hi, max_row + 64, fwd != 0, w_max);
     s.lo = range.lo;
     s.span = range.span;
-    bool fast = range.span != 0 && !s.force_exact;
+    // (p_lo > p_hi: every product is zero)
+    bool fast = range.span != 0 && !s.force_exact && p_lo >= range.lo && p_hi < range.lo + range.span;
     const Tiles vtiles = vertex_tiles(vb), etiles = edge_tiles(ec);
     Sweep sw2[2] = {s, s};
     for (int par = 0; par < 2; ++par) {
@@ -1493,26 +1526,21 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         DRESS_CUDA_TRY(cudaGetLastError());
         return Status::Ok();
     };
-    auto enqueue_pair = [&]() -> Status {
-        DRESS_TRY(enqueue(0));
-        return enqueue(1);
-    };
-    if (fast) {
-        if (uniform) count_launch(), k_fast_start<true><<<eg, 256, 0, st>>>(sw2[0]);
-        else         count_launch(), k_fast_start<false><<<eg, 256, 0, st>>>(sw2[0]);
-    }
     // A pair of certified sweeps (up to 36 launches) and its index steps is
-    // captured once into a CUDA graph and replayed.  A fast sweep is two
-    // launches: capturing and instantiating them (0.4 ms) costs more than the
-    // replays save.
+    // captured into a CUDA graph and replayed, from the sweep `at` on.  A fast
+    // sweep is two launches: capturing and instantiating them (0.4 ms) costs more
+    // than the replays save.
     cudaGraphExec_t gexec = nullptr;
     long long pair_launches = 0;
-    if (!fast) {
+    int gpar = 0;                                     // parity of the pair's first sweep
+    auto capture_pair = [&](int at) -> Status {
+        gpar = at & 1;
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
         const long long before = tls_launches;
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            Status cs = enqueue_pair();
+            Status cs = enqueue(gpar);
+            if (cs.ok()) cs = enqueue(gpar ^ 1);
             cudaError_t e = cudaStreamEndCapture(st, &graph);
             if (cs.ok() && e == cudaSuccess && graph && cudaGraphInstantiate(&gexec, graph, 0) != cudaSuccess)
                 gexec = nullptr;
@@ -1522,11 +1550,13 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         pair_launches = tls_launches - before;
         engine().launches -= pair_launches;           // counted per replay below
         tls_launches -= pair_launches;
-    }
+        return Status::Ok();
+    };
     struct GraphGuard {
-        cudaGraphExec_t g;
+        cudaGraphExec_t &g;
         ~GraphGuard() { if (g) cudaGraphExecDestroy(g); }
     } guard{gexec};
+    if (!fast) DRESS_TRY(capture_pair(0));
     unsigned long long hmax[RING];
     int conv = -1, done = 0;
     int chunk = ctx.cfg->fit_chunk > 0 ? (ctx.cfg->fit_chunk < MAX_CHUNK ? ctx.cfg->fit_chunk : MAX_CHUNK) : 8;
@@ -1534,7 +1564,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     double last_delta = 0.0;
     while (done < max_iterations && conv < 0) {
         for (int r = 0; r < chunk / 2; ++r) {
-            if (gexec && !(done & 1)) {
+            if (gexec && (done & 1) == gpar) {
                 count_launch((int)pair_launches);
                 DRESS_CUDA_TRY(cudaGraphLaunch(gexec, st));
             } else {
@@ -1546,11 +1576,13 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         DRESS_CUDA_TRY(counted_memcpy(hmax, d_maxd.get(), RING * sizeof(unsigned long long),
                                        cudaMemcpyDeviceToHost, st));
         int cert = INT_MAX;
+        bool certify = false;
         if (fast) DRESS_CUDA_TRY(counted_memcpy(&cert, d_cert.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
         DRESS_CUDA_TRY(cudaStreamSynchronize(st));
         if (cert < hi) {                  // the sweeps from `cert` on did not run
             hi = std::max(cert, done);
             fast = false;
+            certify = true;
         }
         for (int it = done; it < hi; ++it) {
             double m;
@@ -1559,6 +1591,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
             if (m < epsilon) { conv = it; break; }
         }
         done = hi;
+        if (certify && conv < 0 && done < max_iterations) DRESS_TRY(capture_pair(done));
         // Next chunk: the sweeps that the decay of the last three deltas
         // predicts until the tolerance, plus two, when they decay; else twice
         // the last chunk.  Sweeps past convergence return at once but still

@@ -89,7 +89,8 @@ struct Sweep {
 
 // Per-sweep max|delta| slots form a ring; the sweep index lives in device
 // memory, so every sweep of a chunk is the same launch sequence (certified ones
-// are replayed from a CUDA graph) and the sweeps after convergence return at once.
+// are replayed from a CUDA graph, also where a fit turns to them on the way) and
+// the sweeps after convergence return at once.
 constexpr int RING = 64;
 
 __device__ __forceinline__ bool skipped(const Sweep &s)
@@ -505,7 +506,8 @@ __global__ void __launch_bounds__(EXACT_THR) k_edge_exact(Sweep s)
 // ---- fast sweeps ------------------------------------------------------------------------
 // While every product lies in [PLO, PHI) (fast_range, delta_nabla.cpp), all
 // additions of rounding errors are exact in any order, for any row or edge of
-// the graph, and a sum needs no certificate: two values a partial sum instead
+// the graph (zero products, of edges of weight zero, change no sum), and a sum
+// needs no certificate: two values a partial sum instead
 // of five, nothing to queue.  The edge kernel checks the products it writes;
 // from the sweep after one left the range (cert_from) the certified kernels
 // above run instead.
@@ -662,7 +664,7 @@ __device__ __forceinline__ bool fast_edge(const Sweep &s, int j, int u, int v, d
     s.dn[j] = r;
     if (!UNIF) s.pn[j] = p;
     lmax = fmax(lmax, fabs(dsub(dj, r)));
-    return (unsigned)__double2hiint(p) - s.lo >= s.span;
+    return (unsigned)__double2hiint(p) - s.lo >= s.span && p != 0.0;
 }
 
 // items of class c: GW lanes each, with pairs unless PAIRS is false
@@ -733,16 +735,6 @@ __global__ void __launch_bounds__(FAST_THR, FAST_RESIDENT) k_edge_fast(Sweep s, 
             s.next[0] = it;
         }
     }
-}
-
-// cert_from of the initial products (INT_MAX: all in range)
-template <bool UNIF>
-__global__ void k_fast_start(Sweep s)
-{
-    bool out = false;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < s.E; j += gridDim.x * blockDim.x)
-        out |= (unsigned)__double2hiint(prod<UNIF>(s, j)) - s.lo >= s.span;
-    if (out) atomicMin(s.cert_from, 0);
 }
 
 // ---- launch of one sweep ------------------------------------------------------------

@@ -108,3 +108,21 @@ def test_owner_rows(low, oracle_port):
     e = np.unique(np.sort(e[e[:, 0] != e[:, 1]], axis=1), axis=0)
     e = e[rng.permutation(len(e))].astype(np.int32)
     _fit(oracle_port, int(e.max()) + 1, e[:, 0].copy(), e[:, 1].copy(), max_iterations=5)
+
+
+@pytest.mark.parametrize("zero", [0.0, -0.0])
+def test_zero_weights_keep_the_fast_sweeps(zero, oracle_port):
+    """Zero products change no sum: ten sweeps take the launches that they take
+    without zeros.  A first product outside leaves no sweep to the fast kernels."""
+    n, U, V = graphs.chung_lu(900, 6000, 2.3, 400, seed=3)
+    W = np.random.default_rng(2).uniform(0.5, 2.0, 6000)
+    launches = []
+    for w in (1.0, zero, -0.001):
+        W[::7] = w
+        with db.Graph(n, U, V, W) as g:
+            db.counters(reset=True)
+            db.fit_graph(g, 10, 0.0)
+            launches.append(db.counters()["launches"])
+        _fit(oracle_port, n, U, V, W)
+        _fit(oracle_port, n, U, V, W, np.random.default_rng(3).uniform(0.5, 2.0, n), db.FORWARD)
+    assert launches[0] == launches[1] < launches[2]
