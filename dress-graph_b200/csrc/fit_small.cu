@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <climits>
 #include <chrono>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -35,6 +36,12 @@ constexpr int CLUSTER_MAX_EDGES = 24576;
 // multi-kernel fit gives such rows a warp or a block.
 constexpr int SMALL_MAX_DEG = 256;
 
+// Graphs of more vertices than 16-bit ids name are fitted without the isolated
+// ones, up to these sizes: 2,000 edges of 100,000 vertices 869 us by the
+// multi-kernel fit, 481 so; 4,000 of 262,144 1,250 and 1,056; 8,000 of 262,144
+// 1,238 and 1,485 where few edges share a vertex.
+constexpr int COMPACT_MAX_VERTICES = 1 << 18, COMPACT_MAX_EDGES = 4096;
+
 // The checks of fit_graph's device validation, on the host: rows in order
 // and in range, edge ids and endpoints in range.
 bool small_graph_ok(p_dress_graph_t g, int &maxdeg)
@@ -56,6 +63,48 @@ bool small_graph_ok(p_dress_graph_t g, int &maxdeg)
     return true;
 }
 
+// The fit of a graph's vertices that have a row or an edge, in their order; the
+// others' norms are the root of their own term.
+Status fit_compact(p_dress_graph_t g, int max_iterations, double epsilon, int *iterations, double *delta,
+                   FitStats *stats, const Ctx &ctx, bool &used)
+{
+    const int N = g->N, E = g->E, S = g->adj_offset[N];
+    int maxdeg = 0;
+    if (N > COMPACT_MAX_VERTICES || E > COMPACT_MAX_EDGES || !small_graph_ok(g, maxdeg)) return Status::Ok();
+    std::vector<int> id((size_t)N, 0), vertex, off, tgt((size_t)S), U((size_t)E), V((size_t)E);
+    for (int e = 0; e < E; ++e) id[(size_t)g->U[e]] = id[(size_t)g->V[e]] = 1;
+    for (int u = 0; u < N; ++u) {
+        if (!id[(size_t)u] && g->adj_offset[u + 1] == g->adj_offset[u]) continue;
+        id[(size_t)u] = (int)vertex.size();
+        vertex.push_back(u);
+        off.push_back(g->adj_offset[u]);
+    }
+    const int n = (int)vertex.size();
+    if (n > UINT16_MAX) return Status::Ok();
+    off.push_back(S);
+    for (int q = 0; q < S; ++q) tgt[(size_t)q] = id[(size_t)g->adj_target[q]];
+    for (int e = 0; e < E; ++e) {
+        U[(size_t)e] = id[(size_t)g->U[e]];
+        V[(size_t)e] = id[(size_t)g->V[e]];
+    }
+    std::vector<double> norms((size_t)n), nw;
+    if (g->NW)
+        for (int u : vertex) nw.push_back(g->NW[u]);
+    dress_graph_t h = *g;
+    h.N = n;
+    h.U = U.data();
+    h.V = V.data();
+    h.adj_offset = off.data();
+    h.adj_target = tgt.data();
+    h.NW = g->NW ? nw.data() : nullptr;
+    h.vertex_dress = norms.data();
+    DRESS_TRY(fit_small(&h, max_iterations, epsilon, iterations, delta, stats, ctx, used));
+    if (!used || max_iterations <= 0) return Status::Ok();
+    for (int u = 0; u < N; ++u) g->vertex_dress[u] = std::sqrt(4.0 * (g->NW ? g->NW[u] : 1.0));
+    for (int i = 0; i < n; ++i) g->vertex_dress[vertex[(size_t)i]] = norms[(size_t)i];
+    return Status::Ok();
+}
+
 }  // namespace
 
 Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *iterations, double *delta,
@@ -69,6 +118,7 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         return Status::Ok();
     const long long S = g->adj_offset[N];
     if (g->adj_offset[0] != 0 || S < 0) return Status::Ok();      // fit_graph reports it
+    if (N > UINT16_MAX) return fit_compact(g, max_iterations, epsilon, iterations, delta, stats, ctx, used);
 
     // one CTA that holds the state and the staged graph, else one cluster
     // whose CTAs hold the values and norms each

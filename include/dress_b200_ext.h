@@ -42,8 +42,11 @@ typedef struct dressx_config_t {
                                      fallback of the certified sums; slower,
                                      same bits); for testing that path        */
     int     one_launch_max_edges; /* graphs up to this many edges are fitted
-                                     in one launch; 0 = built-in limit,
-                                     -1 = never                               */
+                                     in one launch (two where a product is
+                                     out of range); 0 = built-in limit,
+                                     -1 = never.  At most 32,768 edges, 65,535
+                                     slots and 65,535 vertices with an edge
+                                     whatever the value                       */
     int     reserved[6];
 } dressx_config_t;
 

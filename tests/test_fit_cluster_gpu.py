@@ -192,3 +192,23 @@ def test_values_out_of_range_to_go_on_from(oracle_port):
         assert db.counters()["launches"] == 3
         want = np.ctypeslib.as_array(ref.contents.edge_dress, shape=(5003,))
         np.testing.assert_array_equal(g.edge_dress.view(np.int64), want.view(np.int64))
+
+
+@pytest.mark.parametrize("n,N,m", [(3000, 65_536, 2000), (400, 100_000, 900), (4000, 262_144, 4096), (60, 65_536, 1)])
+@pytest.mark.parametrize("variant", [db.UNDIRECTED, db.FORWARD])
+def test_few_edges_among_many_vertices(n, N, m, variant, oracle_port):
+    """More vertices than 16-bit ids, most of them isolated (FORWARD: or without
+    a row of their own): one launch, the isolated ones' norms among the results."""
+    _, U, V = graphs.erdos_renyi(n, m, seed=m)
+    rng = np.random.default_rng(m)
+    at = rng.permutation(N)[:n].astype(np.int32)
+    NW = rng.choice([0.5, 0.5, 0.0, 3.7], N)
+    NW[at] = rng.uniform(0.5, 3.0, n)
+    _fit(oracle_port, N, at[U], at[V], rng.uniform(0.5, 2.0, m), NW, variant)
+    _fit(oracle_port, N, at[U], at[V], None, None, variant, max_iterations=2)
+
+
+@pytest.mark.parametrize("n,N,m", [(3000, 262_145, 2000), (3000, 65_536, 4097)])
+def test_many_vertices_beyond_the_one_launch(n, N, m, oracle_port):
+    _, U, V = graphs.erdos_renyi(n, m, seed=2)
+    _fit(oracle_port, N, U, V, one_launch=False)
