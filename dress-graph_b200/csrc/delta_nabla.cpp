@@ -615,7 +615,7 @@ Status hist_of_host_values(std::vector<Prep *> &ps, cudaStream_t st, int sms)
         o += (long long)p->values_host.size();
     }
     std::vector<std::vector<long long>> out;
-    DRESS_TRY(histogram_segments(keys.get(), alt.get(), begin, len, out, st, sms));
+    DRESS_TRY(histogram_segments(keys.get(), alt.get(), begin, len, out, st));
     for (size_t i = 0; i < ps.size(); ++i) ps[i]->hist = std::move(out[i]);
     return Status::Ok();
 }
@@ -865,7 +865,7 @@ Status exec_batched(BatchPlan &P, const Ctx &en)
             begin[(size_t)i] = P.val_base[(size_t)i];
             len[(size_t)i] = (long long)P.stats[ST_WORDS * (size_t)i + ST_CURSOR];
         }
-        DRESS_TRY(histogram_device(P.d_vals.get(), P.d_alt.get(), begin, len, P.hist, st, en.num_sms));
+        DRESS_TRY(histogram_device(P.d_vals.get(), P.d_alt.get(), begin, len, P.hist, st));
     }
     DRESS_CUDA_TRY(cudaEventRecord(ev[2], st));
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));

@@ -16,7 +16,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <condition_variable>
 #include <vector>
@@ -986,14 +988,64 @@ Status sort_pairs(unsigned long long *keys, unsigned long long *alt, unsigned *v
     return Status::Ok();
 }
 
-Status histogram_device(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
-                        const std::vector<long long> &len, HistResult &res, cudaStream_t st, int sms)
+// Counts and places within a segment take 32 bits: a longer segment is taken in
+// pieces, whose lists are merged on the host (a result of some 10^9 runs would
+// not fit the device beside the values; the usual one of so many values is short).
+constexpr long long SEGMENT_MAX = 1LL << 31;
+
+static Status histogram_pieces(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
+                               const std::vector<long long> &len, HistResult &res, cudaStream_t st)
 {
-    (void)sms;
+    const int nseg = (int)begin.size();
+    std::vector<long long> pb, pl, first;                  // pieces, and every segment's first
+    for (int s = 0; s < nseg; ++s) {
+        first.push_back((long long)pb.size());
+        for (long long o = 0; o < len[(size_t)s]; o += SEGMENT_MAX) {
+            pb.push_back(begin[(size_t)s] + o);
+            pl.push_back(std::min(SEGMENT_MAX, len[(size_t)s] - o));
+        }
+    }
+    first.push_back((long long)pb.size());
+    std::vector<long long> all;
+    try {
+        std::vector<std::vector<long long>> lists;
+        {
+            HistResult part;
+            DRESS_TRY(histogram_device(keys, alt, pb, pl, part, st));
+            DRESS_TRY(histogram_download(part, lists, st));
+        }
+        for (int s = 0; s < nseg; ++s) {
+            std::vector<const int64_t *> p;
+            std::vector<int64_t> n;
+            for (long long i = first[(size_t)s]; i < first[(size_t)s + 1]; ++i) {
+                p.push_back((const int64_t *)lists[(size_t)i].data());
+                n.push_back((int64_t)lists[(size_t)i].size());
+            }
+            int64_t *out = nullptr, out_len = 0;
+            if (dressx_hist_merge(p.data(), n.data(), (int)p.size(), &out, &out_len) != DRESSX_OK) throw std::bad_alloc();
+            const std::unique_ptr<int64_t, void (*)(void *)> own(out, std::free);
+            all.insert(all.end(), out, out + out_len);
+            res.seg_runs[(size_t)s + 1] = (long long)all.size() / 2;
+        }
+    } catch (const std::bad_alloc &) {
+        return Status::Err(DRESSX_ENOMEM, "host allocation of the histograms failed");
+    }
+    res.R = res.seg_runs[(size_t)nseg];
+    DRESS_TRY(res.pairs.alloc(all.size(), st));
+    DRESS_CUDA_TRY(counted_memcpy(res.pairs.get(), all.data(), all.size() * 8, cudaMemcpyHostToDevice, st));
+    DRESS_CUDA_TRY(cudaStreamSynchronize(st));
+    return Status::Ok();
+}
+
+Status histogram_device(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
+                        const std::vector<long long> &len, HistResult &res, cudaStream_t st)
+{
     const int nseg = (int)begin.size();
     res.nseg = nseg;
     res.R = 0;
     res.seg_runs.assign((size_t)nseg + 1, 0);
+    for (long long n : len)
+        if (n > SEGMENT_MAX) return histogram_pieces(keys, alt, begin, len, res, st);
     // descriptors of the launch, packed into one upload
     std::vector<Bucket> bk;
     std::vector<LongSeg> segs;
@@ -1006,7 +1058,6 @@ Status histogram_device(unsigned long long *keys, unsigned long long *alt, const
         const long long b = begin[(size_t)s], n = len[(size_t)s];
         seg_bk[(size_t)s] = (int)bk.size();
         if (n <= 0) continue;
-        if (n >= (1LL << 32)) return Status::Err(DRESSX_EUNSUPPORTED, "histogram segment of 2^32 values or more");
         if (n <= BUCKET_CAP) {
             bk.push_back({b, (unsigned)n, 0u, 1, 0});
             continue;
@@ -1231,10 +1282,10 @@ Status histogram_download(HistResult &res, std::vector<std::vector<long long>> &
 
 Status histogram_segments(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
                           const std::vector<long long> &len, std::vector<std::vector<long long>> &out,
-                          cudaStream_t st, int sms)
+                          cudaStream_t st)
 {
     HistResult res;
-    DRESS_TRY(histogram_device(keys, alt, begin, len, res, st, sms));
+    DRESS_TRY(histogram_device(keys, alt, begin, len, res, st));
     return histogram_download(res, out, st);
 }
 

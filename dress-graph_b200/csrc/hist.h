@@ -19,7 +19,7 @@ struct HistResult {
 // keys: the segments' values (raw double bits), overwritten; alt: scratch of
 // the same size, the same indices.
 Status histogram_device(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
-                        const std::vector<long long> &len, HistResult &res, cudaStream_t st, int sms);
+                        const std::vector<long long> &len, HistResult &res, cudaStream_t st);
 Status histogram_download(HistResult &res, std::vector<std::vector<long long>> &out, cudaStream_t st);
 // Same results straight into malloc'd per-segment arrays (outs[s], lens[s]
 // int64 entries; NULL and 0 for an empty segment; the caller frees them),
@@ -47,6 +47,6 @@ Status segmented_sort(unsigned long long *keys, unsigned long long *alt, const s
 // by value.  `alt` is scratch of the same size as `keys`; both are overwritten.
 Status histogram_segments(unsigned long long *keys, unsigned long long *alt, const std::vector<long long> &begin,
                           const std::vector<long long> &len, std::vector<std::vector<long long>> &out,
-                          cudaStream_t st, int sms);
+                          cudaStream_t st);
 
 }  // namespace dress

@@ -707,7 +707,7 @@ Status collect_batch(Server *sv, Req *r, Ctx *ctx)
     DRESS_TRY(alt.alloc((size_t)n, ctx->st));
     HistResult res;
     DRESS_TRY(histogram_device(r->d_values.get(), alt.get(), std::vector<long long>{0}, std::vector<long long>{n}, res,
-                               ctx->st, sv->sms));
+                               ctx->st));
     std::vector<int64_t *> outs;
     std::vector<long long> lens;
     // at most 8 copy threads: lanes and other finishers share the host

@@ -142,3 +142,30 @@ def test_segments_of_every_size_at_once(oracle_port):
         o.close()
 
 
+
+
+def _shares(g, n, k, parts, **kw):
+    """The histogram of a request and the merged ones of its strided shares."""
+    from dress_b200 import shard
+    whole, _, _, fits, _ = db.hist_requests([g], db.DELTA, k, **kw)[0]
+    flats = [db.hist_requests([g], db.DELTA, k, offset=i, stride=parts, **kw)[0][0] for i in range(parts)]
+    return whole, shard.merge_hists(flats), fits
+
+
+@pytest.mark.slow
+def test_a_segment_of_more_values_than_32_bits_count():
+    """Delta^2 of a circulant graph of 1,000 vertices and 9,000 edges: 4.5*10^9
+    values, taken in pieces.  Each of its three shares is one piece."""
+    import torch
+    if torch.cuda.mem_get_info()[0] < 120 << 30:
+        pytest.skip("needs 85 GB of device memory")
+    n = 1000
+    U = np.tile(np.arange(n, dtype=np.int32), 9)
+    V = np.concatenate([(np.arange(n) + c) % n for c in range(1, 10)]).astype(np.int32)
+    g = db.Graph(n, U, V)
+    whole, merged, fits = _shares(g, n, 2, 3, max_iterations=2)
+    assert fits == n * (n - 1) // 2
+    assert int(whole[1::2].sum()) == fits * 9 * n - sum(2 * 18 - (1 if min(d, n - d) < 10 else 0)
+                                                          for d in range(1, n)) * n // 2
+    np.testing.assert_array_equal(whole, merged)
+    g.close()
