@@ -152,6 +152,18 @@ def _shares(g, n, k, parts, **kw):
     return whole, shard.merge_hists(flats), fits
 
 
+@pytest.mark.parametrize("n,parts", [(140, 4), (200, 24), (300, 80)])
+def test_long_segments_of_distinct_values(n, parts):
+    """6.6, 19.5 and 66 million mostly distinct values: 4,096 buckets of which
+    few, a part and nearly all are more than a block holds.  The shares have at
+    most two million values, with buckets that a block holds."""
+    g = db.Graph(*graphs.random_regular(n, 10, seed=9))
+    whole, merged, _ = _shares(g, n, 2, parts, max_iterations=4)
+    assert whole.size > 10_000_000
+    np.testing.assert_array_equal(whole, merged)
+    g.close()
+
+
 @pytest.mark.slow
 def test_a_segment_of_more_values_than_32_bits_count():
     """Delta^2 of a circulant graph of 1,000 vertices and 9,000 edges: 4.5*10^9
