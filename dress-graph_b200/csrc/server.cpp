@@ -56,9 +56,10 @@ double ms_between(Clock::time_point a, Clock::time_point b)
 
 // Opt-in shared memory per block of a B200 (used when no device is asked).
 constexpr long long B200_SMEM_OPTIN = 232448;
-// Device bytes per value of a histogram: the values, the sort's second
-// buffer, and the sort / run-length scratch.
-constexpr long long HIST_BYTES_PER_VALUE = 56;
+// Device bytes per value of a histogram (histogram_device): the values and their
+// second buffer, 8 each, bucket ids of 2, at most 16 of runs, and less than 1 of
+// buckets, tiles and counters.
+constexpr long long HIST_BYTES_PER_VALUE = 36;
 
 // Pinned staging per lane and finisher at start-up (each grows on demand).
 constexpr size_t STAGE_START_BYTES = (size_t)64 << 20;

@@ -84,3 +84,13 @@ def test_malformed_requests_are_refused():
         else:
             raise AssertionError("accepted an out-of-range endpoint")
         g.ptr.contents.U[2] = U[2]
+
+
+def test_a_histogram_reserves_what_it_takes():
+    # 8 bytes a value twice, 2 of bucket ids, at most 16 of runs, and little else
+    n, U, V = graphs.random_regular(200, 10, seed=1)
+    with db.Graph(n, U, V) as g:
+        for k in (1, 2):
+            values = n * (n - 1) // 2 * 1000 if k == 2 else n * 1000
+            per_value = db.estimate(g, db.DELTA, k)[0] / values
+            assert 34 <= per_value < 37
