@@ -93,7 +93,7 @@ enum { ST_CURSOR = 0, ST_SWEEPS, ST_EDGE_ITERS, ST_FITS, ST_ITERATIONS, ST_DELTA
 // pointer addresses device memory owned by the request, so requests of one
 // launch may live in unrelated allocations.
 struct ParentDesc {
-    int N, E, S, T;
+    int N, E;
     int kind;            // ITEM_*
     int k;
     int fwd;             // FORWARD/BACKWARD self term
@@ -174,7 +174,7 @@ __host__ __device__ inline Geometry chunk_geometry(int N, int E, int k, const Im
     q.staged = gin > 0 && 2 * gin >= gout;
     q.groups = q.staged ? gin : gout;
     q.image = q.staged ? image : 0;
-    if (q.groups < 1) q.groups = 1;          // the launcher refuses states beyond the room
+    if (q.groups < 1) q.groups = 1;          // (the callers have checked that one state fits)
     q.warps = cta / q.groups;
     if (q.warps > 1 && q.groups > 15) q.warps = 1;
     const int useful = (E + 31) / 32 > warps ? (E + 31) / 32 : warps;
@@ -226,8 +226,7 @@ ImageShape plan_products(double nw_min, double nw_max, long long most, bool fwd,
 // The same for the cluster fit (max_deg: the longest row).
 ImageShape plan_cluster(p_dress_graph_t g, int max_deg);
 void pack_cluster(p_dress_graph_t g, const ImageShape &s, unsigned char *dst);
-// Chunks of a launch: parent p's items, divided so that every SM has work
-// (limit >= 0: only the first `limit` items of the whole batch).
+// Chunks of a launch: the parents' items, divided so that every SM has work.
 struct ChunkSource {
     int parent, N, E, k;
     long long first, items;

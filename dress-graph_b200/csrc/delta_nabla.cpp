@@ -403,7 +403,7 @@ inline int next_pow2(int x)
 struct Prep {
     dressx_hist_request_t *r = nullptr;
     p_dress_graph_t g = nullptr;
-    int N = 0, E = 0, S = 0, T = 0;
+    int N = 0, E = 0;
     long long total = 0;               // C(N,k) or P(N,k)
     long long per = 0;                 // ranks in this stride
     std::vector<long long> ranks;      // sampled ranks (empty = all of the stride)
@@ -413,7 +413,7 @@ struct Prep {
     bool batchable = false;
     std::vector<int> ioff, pairs;      // common-neighbour pairs (parent numbering)
     ImageShape img;                    // shape of the packed image
-    int M = 0;
+    int row = 0;                       // longest row (a class of powers of two)
     double *ms_host = nullptr;         // multiset matrix (caller owns after return)
     std::vector<long long> values_host;  // per-subgraph path: values collected on the host
     std::vector<long long> hist;       // flat [bits, count]
@@ -432,7 +432,6 @@ Status prepare(Prep &p)
     p.g = g;
     p.N = g->N;
     p.E = g->E;
-    p.S = g->N > 0 ? g->adj_offset[g->N] : 0;
     const int k = r->k;
     p.total = k == 0 ? 1 : (r->kind == DRESSX_DELTA ? binom_h(p.N, k) : perm_h(p.N, k));
     r->num_subgraphs = p.total;
@@ -474,8 +473,7 @@ Status prepare(Prep &p)
     int maxdeg = 0;
     bool dup = false;
     merge_walk_pairs(g, p.ioff, p.pairs, maxdeg, dup);
-    p.T = p.ioff[(size_t)p.E];
-    p.M = std::max(2, next_pow2(maxdeg + 1));
+    p.row = std::max(2, next_pow2(maxdeg + 1));
     // Masks reproduce the rebuilt subgraph except for the reciprocal-weight
     // lookup of DIRECTED graphs with repeated directed edges.
     // The batch kernel also needs one subgraph's state in shared memory;
@@ -596,7 +594,7 @@ Status run_per_fit(Prep &p, const Ctx &ctx)
 }
 
 // ---- histogram of host-collected values (in-place fits, per-subgraph path) -------
-Status hist_of_host_values(std::vector<Prep *> &ps, cudaStream_t st, int sms)
+Status hist_of_host_values(std::vector<Prep *> &ps, cudaStream_t st)
 {
     long long total = 0;
     for (Prep *p : ps) total += (long long)p->values_host.size();
@@ -630,28 +628,28 @@ struct Tune {
 
 // Size class of a batch, for the schedules that the autotuner measured.
 struct TuneKey {
-    int e, n, M, k;
+    int e, n, row, k;
     bool operator<(const TuneKey &o) const
     {
-        return e != o.e ? e < o.e : n != o.n ? n < o.n : M != o.M ? M < o.M : k < o.k;
+        return e != o.e ? e < o.e : n != o.n ? n < o.n : row != o.row ? row < o.row : k < o.k;
     }
 };
 std::mutex g_tuned_mu;
 std::map<TuneKey, Tune> g_tuned;    // size class -> measured best schedule
 
-TuneKey tune_key(int maxE, int maxN, int M, int maxk)
+TuneKey tune_key(int maxE, int maxN, int row, int maxk)
 {
-    return {next_pow2(maxE), next_pow2(maxN), M, maxk};
+    return {next_pow2(maxE), next_pow2(maxN), row, maxk};
 }
 
 // One warp per subgraph and two CTAs to an SM unless the autotuner has
 // measured the size class: where memory holds fewer subgraphs than warps, the
 // kernel gives each more of them (chunk_geometry).
-Tune pick_tune(int maxE, int maxN, int M, int maxk, const dressx_config_t &cfg)
+Tune pick_tune(int maxE, int maxN, int row, int maxk, const dressx_config_t &cfg)
 {
     if (cfg.group_threads > 0) return {cfg.group_threads};
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    auto it = g_tuned.find(tune_key(maxE, maxN, M, maxk));
+    auto it = g_tuned.find(tune_key(maxE, maxN, row, maxk));
     return it != g_tuned.end() ? it->second : Tune{32};
 }
 
@@ -659,7 +657,7 @@ Tune pick_tune(int maxE, int maxN, int M, int maxk, const dressx_config_t &cfg)
 struct BatchPlan {
     std::vector<Prep *> ps;
     BatchLaunch L{};
-    int maxE = 1, maxN = 1, maxk = 1, M = 2;
+    int maxE = 1, maxN = 1, maxk = 1, row = 2;
     long long max_state = 0;                 // largest smallest-form state of the batch
     int gsize = 32;                          // threads per subgraph, at least
     std::vector<ParentDesc> descs;
@@ -731,11 +729,11 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
         P.maxE = std::max(P.maxE, p->E);
         P.maxN = std::max(P.maxN, p->N);
         P.maxk = std::max(P.maxk, p->r->k);
-        P.M = std::max(P.M, p->M);
+        P.row = std::max(P.row, p->row);
         P.max_state = std::max(P.max_state, state_bytes(p->E, p->N, p->r->k, STATE_VALUE));
         ParentDesc d{};
         d.img = p->img;
-        d.N = p->N; d.E = p->E; d.S = p->S; d.T = p->T;
+        d.N = p->N; d.E = p->E;
         d.kind = p->r->kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA;
         d.k = p->r->k;
         d.fwd = p->g->variant == DRESS_VARIANT_FORWARD || p->g->variant == DRESS_VARIANT_BACKWARD;
@@ -755,7 +753,7 @@ Status plan_batched(std::vector<Prep *> &ps, const Ctx &en, BatchPlan &P)
         if (p->ms_host) ms_total += p->total * (long long)p->E;
     }
     bool fits = false;
-    DRESS_TRY(shape_launch(P, en, pick_tune(P.maxE, P.maxN, P.M, P.maxk, *en.cfg), fits));
+    DRESS_TRY(shape_launch(P, en, pick_tune(P.maxE, P.maxN, P.row, P.maxk, *en.cfg), fits));
     if (!fits) return Status::Err(DRESSX_EUNSUPPORTED, "subgraph state exceeds shared memory");
     BatchLaunch &L = P.L;
 
@@ -997,7 +995,7 @@ Status autotune_batched(BatchPlan &P, const Ctx &en, int *best_out, std::vector<
     if (best < 0) return Status::Err(DRESSX_EUNSUPPORTED, "autotune: no group size fits");
     {
         std::lock_guard<std::mutex> lk(g_tuned_mu);
-        g_tuned[tune_key(P.maxE, P.maxN, P.M, P.maxk)] = best_tu;
+        g_tuned[tune_key(P.maxE, P.maxN, P.row, P.maxk)] = best_tu;
     }
     bool fits = false;
     DRESS_TRY(shape_launch(P, en, best_tu, fits));
@@ -1132,7 +1130,7 @@ Status hist_batch_core(dressx_hist_request_t *reqs, int n, bool per_fit, const C
         std::vector<Prep *> hv;
         for (Prep *p : host_vals)
             if (p->r->want_histogram) hv.push_back(p);
-        Status s = hist_of_host_values(hv, ctx.st, ctx.num_sms);
+        Status s = hist_of_host_values(hv, ctx.st);
         if (!s.ok()) {
             for (Prep *p : hv) p->r->status = s.code;
             if (first.ok()) first = s;

@@ -183,8 +183,6 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         ParentDesc P{};
         P.N = N;
         P.E = E;
-        P.S = (int)S;
-        P.T = (int)T;
         P.kind = ITEM_PLAIN;
         P.k = 0;
         P.fwd = fwd;

@@ -84,7 +84,7 @@ struct Planned {
     int item_kind = ITEM_PLAIN;
     long long items = 0;                // fits to run on the batch path
     long long num_subgraphs = 0;
-    int N = 0, E = 0, S = 0, T = 0, k = 0;
+    int N = 0, E = 0, k = 0;
     int fwd = 0;
     ImageShape img;
     std::vector<unsigned char> packed;  // batch path: the parent image
@@ -124,10 +124,9 @@ Status plan_request(p_dress_graph_t g, int kind, int k, long long smem_cap, bool
     if (kind != DRESSX_FIT && kind != DRESSX_DELTA && kind != DRESSX_NABLA)
         return Status::Err(DRESSX_EINVAL, "bad request kind");
     if (kind != DRESSX_FIT && k < 0) return Status::Err(DRESSX_EINVAL, "negative k");
-    const int N = g->N, E = g->E, S = N > 0 ? g->adj_offset[N] : 0;
+    const int N = g->N, E = g->E;
     pl.N = N;
     pl.E = E;
-    pl.S = S;
     pl.k = kind == DRESSX_FIT ? 0 : k;
     for (int e = 0; e < E; ++e)
         if (g->U[e] < 0 || g->U[e] >= N || g->V[e] < 0 || g->V[e] >= N)
@@ -170,7 +169,6 @@ Status plan_request(p_dress_graph_t g, int kind, int k, long long smem_cap, bool
     }
 
     pl.path = DRESSX_PATH_BATCH;
-    pl.T = (int)(pairs.size() / 2);
     pl.fwd = g->variant == DRESS_VARIANT_FORWARD || g->variant == DRESS_VARIANT_BACKWARD;
     pl.item_kind = kind == DRESSX_FIT ? ITEM_PLAIN : kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA;
     pl.items = kind == DRESSX_FIT ? 1 : pl.num_subgraphs;
@@ -571,8 +569,6 @@ Status Server::admit_batch(Req *r)
     d = ParentDesc{};
     d.N = pl.N;
     d.E = pl.E;
-    d.S = pl.S;
-    d.T = pl.T;
     d.kind = pl.item_kind;
     d.k = pl.k;
     d.fwd = pl.fwd;
@@ -675,7 +671,7 @@ void Server::scheduler()
 }
 
 // ---- finishers and lanes ---------------------------------------------------------
-Status collect_batch(Server *sv, Req *r, Ctx *ctx)
+Status collect_batch(Req *r, Ctx *ctx)
 {
     dressx_server_request_t *p = r->pub;
     const Planned &pl = r->pl;
@@ -738,7 +734,7 @@ void Server::fin_main(Ctx *ctx)
         } else if (r->cancelled) {
             status = DRESSX_ECANCELLED;
         } else {
-            Status s = collect_batch(this, r, ctx);
+            Status s = collect_batch(r, ctx);
             if (!s.ok()) {
                 set_last_error(s);
                 status = s.code;
