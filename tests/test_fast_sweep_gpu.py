@@ -126,3 +126,22 @@ def test_zero_weights_keep_the_fast_sweeps(zero, oracle_port):
         _fit(oracle_port, n, U, V, W)
         _fit(oracle_port, n, U, V, W, np.random.default_rng(3).uniform(0.5, 2.0, n), db.FORWARD)
     assert launches[0] == launches[1] < launches[2]
+
+
+@pytest.mark.parametrize("joins", [2, 7])
+def test_owner_rows_beyond_the_ranked(joins, oracle_port):
+    """More than 2^20 edges and an oriented row of more than 1,024: that row keeps
+    its order in the renumbering by owner.  With seven permutations of the core
+    joined the triangles overflow their list, and a second pass makes the pairs."""
+    low = 1100
+    rng = np.random.default_rng(joins)
+    core = np.arange(1, low + 1)
+    far = np.arange(low + 1, 2 * low + 41)
+    e = [np.stack([np.zeros(low, int), core], 1)]
+    e += [np.stack([np.full(low + 1, c), rng.choice(far, low + 1, replace=False)], 1) for c in core]
+    e += [np.stack([core, rng.permutation(core)], 1) for _ in range(joins)]
+    e = np.concatenate(e)
+    e = np.unique(np.sort(e[e[:, 0] != e[:, 1]], axis=1), axis=0)
+    e = e[rng.permutation(len(e))].astype(np.int32)
+    assert len(e) > 1 << 20
+    _fit(oracle_port, int(e.max()) + 1, e[:, 0].copy(), e[:, 1].copy(), rng.uniform(0.5, 2.0, len(e)), max_iterations=1)

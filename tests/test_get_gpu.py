@@ -68,7 +68,7 @@ def test_power_law_pairs(exact, oracle_port):
     _check(oracle_port, n, U, V, None, q)
 
 
-@pytest.mark.parametrize("run,other", [(31, 33), (64, 40), (1000, 999), (4000, 4100)])
+@pytest.mark.parametrize("run,other", [(31, 33), (64, 40), (1000, 999), (1500, 1600)])
 def test_long_runs_of_parallel_edges(run, other, oracle_port):
     """Runs within, across and far beyond a warp's strip, of unequal length in
     the two rows; the place in a run is found by search, not step by step."""

@@ -228,3 +228,26 @@ def test_served_large_histogram_equals_direct_call():
         assert r["status"] == 0
         np.testing.assert_array_equal(r["hist_flat"], direct)
         assert direct.size * 8 > 64 << 20
+
+
+@pytest.mark.parametrize("m", [1025, 1500, 2047, 2048])
+@pytest.mark.parametrize("weights", ["none", "uniform", "one to ten", "zeros"])
+def test_whole_graph_items_of_the_batch_kernel(m, weights, oracle_port):
+    """Fits above the one-CTA limit that the server still packs into batch
+    launches, alone and all at once, with vertex weights."""
+    rng = np.random.default_rng(m)
+    n, U, V = graphs.erdos_renyi(m // 3, m, seed=m)
+    W = {"none": None, "uniform": rng.uniform(0.5, 2.0, m), "one to ten": rng.integers(1, 11, m).astype(float),
+         "zeros": rng.integers(0, 3, m).astype(float)}[weights]
+    NWs = [None, rng.uniform(0.1, 3.0, n)]
+    with db.Server() as srv:
+        gs = [db.Graph(n, U, V, W, NW) for NW in NWs for _ in range(3)]
+        tickets = [srv.submit(g) for g in gs]
+        for i, (g, t) in enumerate(zip(gs, tickets)):
+            r = t.wait()
+            ref = oracle_port.fit(n, U, V, W, NWs[i // 3])
+            assert r["status"] == 0 and r["path"] == db.PATH_BATCH
+            assert (r["iterations"], r["delta"]) == (ref["iterations"], ref["delta"])
+            np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
+            np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
+            g.close()
