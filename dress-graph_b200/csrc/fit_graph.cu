@@ -1419,8 +1419,8 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // The edge arrays in the new numbering.  Nothing above reads them when the
     // triangle listing made the pairs, so all of it runs beside their upload
-    // (28 M edges: the set-up ends 33 ms after the call began, 44 when the
-    // renumbering waited for the edge arrays).
+    // (28 M edges: the set-up ends 32 to 41 ms after the call began, 42 to 47 when
+    // the renumbering waited for the edge arrays).
     if (!edges_valid) DRESS_TRY(validate_edges());
     DRESS_TRY(d_nwi.alloc((size_t)N, st));
     DRESS_TRY(d_eu.alloc((size_t)E, st));
