@@ -100,3 +100,23 @@ def test_zero_weights_among_others(n, m, oracle_port):
         assert (it, delta) == (ref["iterations"], ref["delta"])
         np.testing.assert_array_equal(g.edge_dress.view(np.int64), ref["edge_dress"].view(np.int64))
         np.testing.assert_array_equal(g.vertex_dress.view(np.int64), ref["vertex_dress"].view(np.int64))
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 1e300, 5e-324])
+@pytest.mark.parametrize("m", [100, 900, 3000, 30_001])
+def test_weights_without_a_finite_sum(m, bad, oracle_port):
+    """A NaN term, which sorts nowhere, makes its sum NaN on every path: one CTA,
+    cluster, multi-kernel and the subgraphs of a batch."""
+    n, U, V = graphs.erdos_renyi(max(30, m // 5), m, seed=m)
+    W = np.random.default_rng(1).uniform(0.5, 2.0, m)
+    W[[3, m // 2]] = bad
+    ref = oracle_port.fit(n, U, V, W)
+    with db.Graph(n, U, V, W) as g:
+        it, delta = db.fit_graph(g)
+        assert (it, delta) == (ref["iterations"], ref["delta"])
+        np.testing.assert_array_equal(bits(g.edge_dress), bits(ref["edge_dress"]))
+        np.testing.assert_array_equal(bits(g.vertex_dress), bits(ref["vertex_dress"]))
+    if m < 1000 and not np.isnan(bad):
+        with db.Graph(n, U, V, W) as g:
+            flat = db.hist_requests([g], db.DELTA, 1, n_samples=8, seed=1)[0][0]
+        np.testing.assert_array_equal(flat, oracle_port.delta_fit(n, U, V, W, k=1, n_samples=8, seed=1)["hist"])
