@@ -58,7 +58,8 @@ __device__ __forceinline__ unsigned lanemask_lt()
 // flags[0]: malformed input, flags[1]: a row repeats a neighbour,
 // flags[2]: edge weights are not all bit-identical, flags[3]: max row length,
 // flags[4..5]: the largest positive weight (bits of the double), flags[6]: an
-// edge id stands in two oriented slots (k_slot_counts), flags[8..11]:
+// edge id stands in two oriented slots (k_slot_counts), flags[7]: most pairs of
+// an edge in the graph's own tables (k_given_counts), flags[8..11]:
 // the smallest and largest vertex weight (k_nw_bounds), flags[12..13]: the
 // complement of the smallest and the largest high word of the first products
 // w*d that are not zero.
@@ -176,11 +177,20 @@ __global__ void k_nw_bounds(int N, const double *nw, unsigned long long *lohi)
 // ---- intercepts from the graph's own tables ----
 __global__ void k_given_counts(int E, const int *io, int *cnt, int *flags)
 {
+    __shared__ int block_most;
+    if (threadIdx.x == 0) block_most = 0;
+    __syncthreads();
+    int most = 0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
         int c = io[e + 1] - io[e];
         if (c < 0) { atomicOr(&flags[0], 16); c = 0; }
         cnt[e] = c;
+        most = max(most, c);
     }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(&block_most, most);
+    __syncthreads();
+    if (threadIdx.x == 0 && block_most > 0) atomicMax(&flags[7], block_most);
 }
 
 __global__ void k_given_pairs(int E, const int *io, const int *ux, const int *vx,
@@ -1196,6 +1206,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     DRESS_CUDA_TRY(cudaStreamSynchronize(st));
     const double t_pairs = ms_since(t0), early_ms = edge_up.wait_ms + t_valid;   // (part of it)
     if (flags[0]) return Status::Err(DRESSX_EINVAL, "malformed intercept tables");
+    const int most_given = flags[7];
     // fine ranges (cursors), then the coarse bins they make up
     std::vector<int> cur(2 * NF);
     cur[0] = 0;
@@ -1442,7 +1453,10 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     int smem_optin = 0;
     DRESS_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
     const int exact_cap = (smem_optin - 2048) / 8;
-    const long long max_terms = max_row + 1;       // a row's slots or an edge's pairs, plus the self term
+    // a row's slots or an edge's pairs; a graph's own tables may hold more pairs
+    // than any row has slots
+    const long long longest = std::max<long long>(max_row, most_given);
+    const long long max_terms = longest + 1;       // and the self term
     const int exact_grid = max_terms > exact_cap ? std::min(32, 2 * sms) : 2 * sms;
     DevBuf<double> d_scratch;
     long long scratch_stride = 0;
@@ -1498,7 +1512,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     s.iter = s.next = d_iter.get();
     s.max_iter = max_iterations;
     // the range of products in which sums need no certificate, for this
-    // graph's longest row (no edge has more pairs)
+    // graph's longest row or list of pairs
     DevBuf<int> d_cert;
     DRESS_TRY(d_cert.alloc(1, st));
     {
@@ -1506,7 +1520,7 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
         DRESS_CUDA_TRY(counted_memcpy(d_cert.get(), &never, sizeof(int), cudaMemcpyHostToDevice, st));
     }
     s.cert_from = d_cert.get();
-    const ImageShape range = plan_products(nw_lo, nw_hi, max_row + 64, fwd != 0, w_max);
+    const ImageShape range = plan_products(nw_lo, nw_hi, longest + 64, fwd != 0, w_max);
     s.lo = range.lo;
     s.span = range.span;
     // (p_lo > p_hi: every product is zero)

@@ -9,6 +9,8 @@ the oracle: the single-graph fit (shared-memory sorts and, for a hub beyond
 shared memory, the global-scratch sort), the one-launch fits and the
 batched Delta/Nabla kernel (its in-place selection order).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -120,3 +122,44 @@ def test_weights_without_a_finite_sum(m, bad, oracle_port):
         with db.Graph(n, U, V, W) as g:
             flat = db.hist_requests([g], db.DELTA, 1, n_samples=8, seed=1)[0][0]
         np.testing.assert_array_equal(flat, oracle_port.delta_fit(n, U, V, W, k=1, n_samples=8, seed=1)["hist"])
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("pairs", [1, 40, 600, 30_000, 70_001])
+def test_own_tables_longer_than_the_rows(pairs, exact, oracle_port):
+    """A caller's tables may list more pairs for an edge than any row has slots:
+    up to and beyond what a block sorts in shared memory."""
+    n = 40
+    U, V = np.arange(n - 1, dtype=np.int32), np.arange(1, n, dtype=np.int32)
+    rng = np.random.default_rng(pairs)
+    W = rng.uniform(0.5, 2.0, n - 1)
+    off = np.zeros(n, np.int32)
+    off[8:] = pairs                                  # all of them edge 7's
+    ux, vx = (rng.integers(0, n - 1, pairs).astype(np.int32) for _ in range(2))
+    names = ("intercept_offset", "intercept_edge_ux", "intercept_edge_vx")
+    ip = ctypes.POINTER(ctypes.c_int)
+
+    def fitted(c, fit):
+        kept = [ctypes.cast(getattr(c, f), ctypes.c_void_p).value for f in names]
+        c.max_degree = max(2, pairs)                 # what the oracle's buffer is sized by
+        for f, a in zip(names, (off, ux, vx)):
+            setattr(c, f, a.ctypes.data_as(ip))
+        r = fit()
+        for f, p in zip(names, kept):
+            setattr(c, f, ctypes.cast(p, ip))
+        return r, [np.ctypeslib.as_array(getattr(c, f), shape=(k,)).copy()
+                   for f, k in (("edge_dress", n - 1), ("vertex_dress", n))]
+
+    ref = oracle_port.build(n, U, V, W, None, db.UNDIRECTED, 1)
+    it, delta = ctypes.c_int(), ctypes.c_double()
+    _, want = fitted(ref.contents, lambda: oracle_port.fit_fn(ref, 20, 1e-6, ctypes.byref(it), ctypes.byref(delta)))
+    oracle_port.free_graph(ref)
+    db.configure(exact_sums=exact)
+    try:
+        with db.Graph(n, U, V, W, precompute_intercepts=True) as g:
+            got, values = fitted(g.ptr.contents, lambda: db.fit_graph(g, 20))
+    finally:
+        db.configure()
+    assert got == (it.value, delta.value)
+    for a, b in zip(values, want):
+        np.testing.assert_array_equal(bits(a), bits(b))
