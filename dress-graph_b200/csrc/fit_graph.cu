@@ -1525,15 +1525,15 @@ Status fit_graph(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
     s.span = range.span;
     // (p_lo > p_hi: every product is zero)
     bool fast = range.span != 0 && !s.force_exact && p_lo >= range.lo && p_hi < range.lo + range.span;
-    const Tiles vtiles = vertex_tiles(vb), etiles = edge_tiles(ec);
+    const Tiles vtiles = vertex_tiles(vb), ltiles = long_edge_tiles(ec, sms), etiles = edge_tiles(ec, ltiles);
     Sweep sw2[2] = {s, s};
     for (int par = 0; par < 2; ++par) {
         sw2[par].d = dbuf[par]; sw2[par].dn = dbuf[par ^ 1];
         sw2[par].p = pbuf[par]; sw2[par].pn = pbuf[par ^ 1];
     }
     auto enqueue = [&](int par) -> Status {
-        if (fast && uniform) return launch_fast_sweep<true>(sw2[par], vtiles, etiles, lc);
-        if (fast) return launch_fast_sweep<false>(sw2[par], vtiles, etiles, lc);
+        if (fast && uniform) return launch_fast_sweep<true>(sw2[par], vtiles, ltiles, etiles, lc);
+        if (fast) return launch_fast_sweep<false>(sw2[par], vtiles, ltiles, etiles, lc);
         if (uniform) DRESS_TRY(launch_sweep<true>(sw2[par], vb, ec, lc));
         else         DRESS_TRY(launch_sweep<false>(sw2[par], vb, ec, lc));
         count_launch(), k_next_sweep<<<1, 1, 0, st>>>(d_iter.get(), d_maxd.get(), d_qcount.get());

@@ -520,7 +520,11 @@ __global__ void __launch_bounds__(EXACT_THR) k_edge_exact(Sweep s)
 // 1.21 ms with 7 or 8 resident blocks, which spill).
 // Rows and edges of more than MED_CAP terms take a block each: a warp's 128
 // terms a lane made the longest of them the sweep's tail (22 us on the 200,003
-// edges).
+// edges).  Edges of up to BIG_CAP pairs take a warp each where there are eight of
+// them to a resident warp: the tail is then short against the phase, and a block
+// spends its barriers on three terms a thread (K_800, 798 pairs an edge: 1.65 ms
+// a sweep with blocks, 1.0 with warps).  They are a launch of their own, as a
+// seventh class cost the kernel registers (3 % of a sweep at 28 M edges).
 
 // s + c is the exact sum so far
 struct ExactSum {
@@ -737,6 +741,19 @@ __global__ void __launch_bounds__(FAST_THR, FAST_RESIDENT) k_edge_fast(Sweep s, 
     }
 }
 
+// the items of class 1, ahead of k_edge_fast, which ends the sweep
+template <bool UNIF>
+__global__ void __launch_bounds__(FAST_THR, FAST_RESIDENT) k_edge_long(Sweep s, Tiles T)
+{
+    if (fast_skipped(s)) return;
+    double lmax = 0.0;
+    bool out = false;
+    for (int tile = blockIdx.x; tile < T.first[2]; tile += gridDim.x)
+        out |= edge_tile<UNIF, 32, true>(s, T, 1, tile, lmax);
+    if (out) atomicMin(s.cert_from, *s.iter + 1);
+    block_max_to(max_slot(s), lmax);
+}
+
 // ---- launch of one sweep ------------------------------------------------------------
 
 struct Bins {
@@ -886,11 +903,24 @@ inline Tiles vertex_tiles(const Bins &b)
     return T;
 }
 
-inline Tiles edge_tiles(const EdgeClasses &ec)
+// the edges of 513..BIG_CAP pairs where they are a warp each, as class 1
+inline Tiles long_edge_tiles(const EdgeClasses &ec, int sms)
+{
+    Tiles T{};
+    if (ec.cls[5] - ec.cls[4] < 8 * FAST_RESIDENT * (FAST_THR / 32) * sms) return T;
+    T.lo[1] = ec.cls[4];
+    T.hi[1] = ec.cls[5];
+    T.list = ec.list;
+    number_tiles(T);
+    return T;
+}
+
+// the others
+inline Tiles edge_tiles(const EdgeClasses &ec, const Tiles &longs)
 {
     Tiles T{};
     const int *k = ec.cls;
-    const int lo[6] = {k[4], k[1], k[2], k[3], k[0], 0}, hi[6] = {k[6], k[2], k[3], k[4], k[1], ec.e0};
+    const int lo[6] = {longs.first[2] > 0 ? k[5] : k[4], k[1], k[2], k[3], k[0], 0}, hi[6] = {k[6], k[2], k[3], k[4], k[1], ec.e0};
     for (int c = 0; c < 6; ++c) {
         T.lo[c] = lo[c];
         T.hi[c] = hi[c];
@@ -903,13 +933,15 @@ inline Tiles edge_tiles(const EdgeClasses &ec)
 }
 
 template <bool UNIF>
-Status launch_fast_sweep(const Sweep &s, const Tiles &vt, const Tiles &et, const LaunchCfg &c)
+Status launch_fast_sweep(const Sweep &s, const Tiles &vt, const Tiles &lt, const Tiles &et, const LaunchCfg &c)
 {
     const int wave = FAST_RESIDENT * c.sms;
     if (vt.first[5] > 0)
         count_launch(), k_vertex_fast<UNIF><<<std::min(vt.first[5], wave), FAST_THR, 0, c.st>>>(s, vt);
-    if (et.first[6] > 0)
-        count_launch(), k_edge_fast<UNIF><<<std::min(et.first[6], wave), FAST_THR, 0, c.st>>>(s, et);
+    if (lt.first[2] > 0)
+        count_launch(), k_edge_long<UNIF><<<std::min(lt.first[2], wave), FAST_THR, 0, c.st>>>(s, lt);
+    // (also without items of its own: it ends the sweep)
+    count_launch(), k_edge_fast<UNIF><<<std::max(1, std::min(et.first[6], wave)), FAST_THR, 0, c.st>>>(s, et);
     DRESS_CUDA_TRY(cudaGetLastError());
     return Status::Ok();
 }

@@ -145,3 +145,12 @@ def test_owner_rows_beyond_the_ranked(joins, oracle_port):
     e = e[rng.permutation(len(e))].astype(np.int32)
     assert len(e) > 1 << 20
     _fit(oracle_port, int(e.max()) + 1, e[:, 0].copy(), e[:, 1].copy(), rng.uniform(0.5, 2.0, len(e)), max_iterations=1)
+
+
+@pytest.mark.parametrize("n,variant", [(520, db.UNDIRECTED), (330, db.UNDIRECTED), (520, db.FORWARD)])
+def test_many_long_lists_of_pairs(n, variant, oracle_port):
+    """A complete graph: 134,940 edges of 518 pairs are a warp each, 54,285 of
+    328 lane groups as ever."""
+    U, V = (x.astype(np.int32) for x in np.triu_indices(n, 1))
+    W = np.random.default_rng(n).uniform(0.5, 2.0, len(U))
+    _fit(oracle_port, n, U, V, W, variant=variant, max_iterations=2)
