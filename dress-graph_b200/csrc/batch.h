@@ -201,11 +201,15 @@ struct ClusterFit {
 // Whether one CTA's memory holds the values and norms.
 bool cluster_fits(int E, int N, int S);
 Status launch_cluster_fit(const ClusterFit &f, cudaStream_t st);
-// A graph is batchable when one subgraph's smallest state fits.
+// A graph is batchable when one subgraph's smallest state fits and the image can
+// name it: ids below 2^15 and 2^16, at most 65,535 groups of row slots (S slots of
+// rows padded to groups of four).  Rows of two slots an edge stay far below; a
+// caller's own rows may hold more.
 constexpr long long BATCH_STATE_MAX = 227 * 1024 - BATCH_HEADER;
-inline bool batch_fits(int E, int N, int k)
+inline bool batch_fits(int E, int N, long long S, int k)
 {
-    return E < 32768 && N < 65536 && state_bytes(E, N, k, STATE_VALUE) <= BATCH_STATE_MAX;
+    return E < 32768 && N < 65536 && S + 3LL * N <= 4 * 65535LL &&
+           state_bytes(E, N, k, STATE_VALUE) <= BATCH_STATE_MAX;
 }
 
 // ---- host planning helpers (delta_nabla.cpp) ------------------------------------

@@ -510,7 +510,8 @@ Status prepare(Prep &p)
     // lookup of DIRECTED graphs with repeated directed edges.
     // The batch kernel also needs one subgraph's state in shared memory;
     // rows of any length are summed there (certified sums, no networks).
-    p.batchable = !(dup && g->variant == DRESS_VARIANT_DIRECTED) && batch_fits(p.E, p.N, k);
+    p.batchable = !(dup && g->variant == DRESS_VARIANT_DIRECTED) &&
+                  batch_fits(p.E, p.N, p.N > 0 ? g->adj_offset[p.N] : 0, k);
     if (p.batchable) p.img = plan_image(g, p.ioff, r->kind == DRESSX_DELTA ? ITEM_DELTA : ITEM_NABLA, k, false, false);
     return Status::Ok();
 }

@@ -122,7 +122,7 @@ Status fit_small(p_dress_graph_t g, int max_iterations, double epsilon, int *ite
 
     // one CTA that holds the state and the staged graph, else one cluster
     // whose CTAs hold the values and norms each
-    bool one_cta = E <= SMALL_MAX_EDGES && batch_fits(E, N, 0);
+    bool one_cta = E <= SMALL_MAX_EDGES && batch_fits(E, N, S, 0);
     const bool cluster = cluster_fits(E, N, (int)std::min<long long>(S, INT_MAX)) && ctx.cfg->exact_sums == 0;
     if (!one_cta && !cluster) return Status::Ok();
     int maxdeg = 0;

@@ -140,7 +140,8 @@ Status plan_request(p_dress_graph_t g, int kind, int k, long long smem_cap, bool
     // 1 <= k < N (the other orders are trivial or in-place fits, served by
     // the lane path).  A whole-graph fit keeps rows of at most 256
     // neighbours: one thread sums a row there.
-    bool batch = batch_fits(E, N, pl.k) && state_bytes(E, N, pl.k, STATE_VALUE) <= batch_room((int)smem_cap);
+    bool batch = batch_fits(E, N, N > 0 ? g->adj_offset[N] : 0, pl.k) &&
+                 state_bytes(E, N, pl.k, STATE_VALUE) <= batch_room((int)smem_cap);
     if (kind == DRESSX_FIT) batch = batch && maxdeg <= 256;
     if (kind != DRESSX_FIT) batch = batch && k >= 1 && k < N;
     // a whole-graph fit in the batch kernel runs on one thread group (one

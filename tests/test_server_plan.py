@@ -1,6 +1,9 @@
-"""Host-side planning of served requests (no GPU): path choice and the
-device bytes a request reserves at admission."""
+"""Host-side planning of served requests (no GPU, but for one test): path choice
+and the device bytes a request reserves at admission."""
+import ctypes
+
 import numpy as np
+import pytest
 
 import dress_b200 as db
 from dress_b200 import graphs
@@ -94,3 +97,65 @@ def test_a_histogram_reserves_what_it_takes():
             values = n * (n - 1) // 2 * 1000 if k == 2 else n * 1000
             per_value = db.estimate(g, db.DELTA, k)[0] / values
             assert 34 <= per_value < 37
+
+
+def own_rows(c, n, per_row):
+    """Rows of a caller's own for the cycle of n vertices, each neighbour listed
+    per_row / 2 times; returns what puts the graph's rows back."""
+    u = np.arange(n, dtype=np.int32)
+    nbr, eid = np.stack([np.roll(u, 1), np.roll(u, -1)], 1), np.stack([np.roll(u, 1), u], 1)
+    order = np.argsort(nbr, axis=1)
+    tgt, idx = (np.repeat(np.take_along_axis(a, order, 1), per_row // 2, axis=1).ravel() for a in (nbr, eid))
+    rows = {"adj_offset": np.arange(0, n * per_row + 1, per_row, dtype=np.int32),
+            "adj_target": tgt, "adj_edge_idx": idx}
+    ip = ctypes.POINTER(ctypes.c_int)
+    kept = {f: ctypes.cast(getattr(c, f), ctypes.c_void_p).value for f in rows}
+    for f, a in rows.items():
+        setattr(c, f, a.ctypes.data_as(ip))
+    c.max_degree = per_row                               # what the oracle's buffer is sized by
+
+    def back():
+        for f, p in kept.items():
+            setattr(c, f, ctypes.cast(p, ip))
+        return rows
+
+    return back
+
+
+# the batch kernel's image names 65,535 groups of four slots
+ROWS = [(200, db.PATH_BATCH), (216, db.PATH_LANE), (256, db.PATH_LANE)]
+
+
+@pytest.mark.parametrize("per_row, path", ROWS)
+def test_rows_of_more_slots_than_the_image_names(per_row, path):
+    n = 1200
+    U = np.arange(n, dtype=np.int32)
+    with db.Graph(n, U, np.roll(U, -1)) as g:
+        back = own_rows(g.ptr.contents, n, per_row)
+        paths = [db.estimate(g, kind, k)[1] for kind, k in ((db.FIT, 0), (db.DELTA, 1))]
+        back()
+    assert paths == [path, path]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("per_row, path", ROWS)
+def test_served_fit_of_own_rows(per_row, path, oracle_port):
+    n = 1200
+    U = np.arange(n, dtype=np.int32)
+    V = np.roll(U, -1)
+    W = np.random.default_rng(1).uniform(0.5, 2.0, n)
+    ref = oracle_port.build(n, U, V, W, None, db.UNDIRECTED, 0)
+    back = own_rows(ref.contents, n, per_row)
+    it, delta = ctypes.c_int(), ctypes.c_double()
+    oracle_port.fit_fn(ref, 100, 1e-6, ctypes.byref(it), ctypes.byref(delta))
+    want = [np.ctypeslib.as_array(f, shape=(n,)).copy() for f in (ref.contents.edge_dress, ref.contents.vertex_dress)]
+    back()
+    oracle_port.free_graph(ref)
+    with db.Server() as srv, db.Graph(n, U, V, W) as g:
+        back = own_rows(g.ptr.contents, n, per_row)
+        r = srv.submit(g).wait()
+        back()
+        assert r["status"] == 0 and r["path"] == path
+        assert (r["iterations"], r["delta"]) == (it.value, delta.value)
+        for a, b in zip((g.edge_dress, g.vertex_dress), want):
+            np.testing.assert_array_equal(a.view(np.int64), b.view(np.int64))
